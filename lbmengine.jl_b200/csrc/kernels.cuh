@@ -88,7 +88,7 @@ struct ParticleDev {
     int rules;               // LBM_RULES_* of the model: which module's particle update and node velocity
     int recordF;             // accumulate the momentum-exchange force even when coupleF is off (the
                              // adjoint's force observable; the force is reported, never applied)
-    int pad2;
+    int rec_tick;            // records written to ParticleArgs::rec (lbm_adjoint's forward ticks)
     long long nrec;          // ticks recorded into the trajectory ring (ParticleArgs::trj)
 };
 

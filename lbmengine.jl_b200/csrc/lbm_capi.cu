@@ -53,6 +53,10 @@ constexpr int kModelGraphTicks = kModelGraphSizes[0];
 // Later calls build and replay graphs.
 constexpr int kFirstCallDirectTicks = 32;
 static_assert(kFirstCallDirectTicks <= kModelGraphTicks, "profiling slots");
+// lbm_adjoint runs of at least this many ticks build graphs for their forward
+// ticks (one to a few recomputations of every tick repay the build), shorter
+// ones launch them directly.
+constexpr int kAdjointGraphTicks = 256;
 
 }  // namespace
 
@@ -137,6 +141,7 @@ struct lbm_handle {
     // trajectory recording (lbm_record_trajectories): ring of trj_cap ticks
     double* d_trj = nullptr;
     long long trj_cap = 0, trj_read = 0;
+    ParticleDev* d_rec = nullptr;  // particle history of a running lbm_adjoint
     // asynchronous writer of fluid snapshots (lbm_write_fluid_csv)
     std::thread writer;
     std::string writer_err;
@@ -574,6 +579,7 @@ ParticleArgs particle_args(const lbm_handle* h, int mode, int pid, int src = -1)
     a.err = h->d_err;
     a.trj = h->d_trj;
     a.trj_cap = h->trj_cap;
+    a.rec = h->d_rec;
     a.fint = h->inter.empty() ? nullptr : h->d_fint;
     return a;
 }
@@ -2908,69 +2914,11 @@ void lbm_batch_destroy(lbm_batch* b) { batch_destroy_all(b); }
 
 // ===========================================================================
 // Gradients (lbm_adjoint): discrete adjoint of the tick with binomial
-// checkpointing.  Device: the field adjoint (adjoint.cuh).  Host: the
-// particle update's adjoint (a handful of FP64 values per tick) and the
-// checkpoint schedule.
+// checkpointing.  Device: the adjoint of the fields and of the particle update
+// (adjoint.cuh).  Host: the checkpoint schedule, which enqueues forward and
+// backward ticks without waiting for them.
 // ===========================================================================
 namespace {
-
-// forward-mode dual with one direction, host side
-struct HD {
-    double v = 0, d = 0;
-};
-HD operator+(HD a, HD b) { return {a.v + b.v, a.d + b.d}; }
-HD operator-(HD a, HD b) { return {a.v - b.v, a.d - b.d}; }
-HD operator*(HD a, HD b) { return {a.v * b.v, a.d * b.v + a.v * b.d}; }
-HD operator/(HD a, HD b) {
-    const double q = a.v / b.v;
-    return {q, (a.d - q * b.d) / b.v};
-}
-HD operator*(double s, HD a) { return {s * a.v, s * a.d}; }
-HD hsqrt(HD a) {
-    const double r = std::sqrt(a.v);
-    return {r, a.d / (2 * r)};
-}
-HD hcos(HD a) { return {std::cos(a.v), -std::sin(a.v) * a.d}; }
-HD hsin(HD a) { return {std::sin(a.v), std::cos(a.v) * a.d}; }
-HD habs(HD a) { return a.v < 0 ? HD{-a.v, -a.d} : a; }
-
-// the swimming-direction update of moveParticles! (particles.jl:48-70:
-// Rodrigues rotation by |w| dt about w, then normalised), as the particle
-// kernel does it
-void rodrigues(const HD* e, const HD* w, double dt, int D, HD* out) {
-    for (int k = 0; k < 3; ++k) out[k] = e[k];
-    HD theta;
-    if (D == 2) theta = habs(w[0]);
-    else theta = hsqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
-    if (theta.v == 0.0) return;
-    HD vr[3];
-    if (D == 2) {
-        const HD k = w[0] / theta;
-        const HD th = dt * theta;
-        const HD ct = hcos(th), st = hsin(th);
-        vr[0] = e[0] * ct + (HD{0, 0} - k * e[1]) * st;
-        vr[1] = e[1] * ct + (k * e[0]) * st;
-        vr[2] = HD{};
-    } else {
-        const HD k[3] = {w[0] / theta, w[1] / theta, w[2] / theta};
-        const HD th = dt * theta;
-        const HD ct = hcos(th), st = hsin(th);
-        const HD cr[3] = {k[1] * e[2] - k[2] * e[1], HD{0, 0} - k[0] * e[2] + k[2] * e[0], k[0] * e[1] - k[1] * e[0]};
-        const HD kv = k[0] * e[0] + k[1] * e[1] + k[2] * e[2];
-        for (int q = 0; q < 3; ++q) vr[q] = e[q] * ct + cr[q] * st + k[q] * kv * (HD{1, 0} - ct);
-    }
-    HD n2{};
-    for (int q = 0; q < D; ++q) n2 = n2 + vr[q] * vr[q];
-    const HD nr = hsqrt(n2);
-    for (int q = 0; q < D; ++q) out[q] = vr[q] / nr;
-}
-
-// adjoint of the particle state carried backwards through the ticks
-struct PartAdj {
-    double R[3] = {0, 0, 0}, v[3] = {0, 0, 0}, w[3] = {0, 0, 0}, e[3] = {0, 0, 0};
-    double S[12] = {0};  // snapshot sR, sV, sW, sE
-    double mR[3] = {0, 0, 0};
-};
 
 struct Snap {
     char* buf = nullptr;
@@ -2981,50 +2929,77 @@ struct Snap {
 
 struct AdjointRun {
     lbm_handle* h = nullptr;
-    lbm_adjoint_spec spec{};
-    std::vector<ParticleDev> rec;  // rec[t]: the particle after t ticks
-    std::vector<char> have;        // rec[t] has been recorded
+    AdjArgs args{};                // of the backward kernels; src, lam and n set per tick
+    std::vector<char> have;        // have[t]: the particle after t ticks is in the device history
     std::vector<Snap> snaps;       // stored states (a stack)
+    std::vector<char*> spare;      // free buffers: pieces of one block, then what was allocated one by one
+    std::vector<char*> extra;
     size_t snap_bytes = 0;
     int max_used = 0;
     long long forward = 0;
     double* lam[2] = {nullptr, nullptr};
     int lcur = 0;  // lam[lcur]: adjoint of the populations at the current tick
-    double* partial = nullptr;
-    double* dsum = nullptr;
-    long long nblocks = 0;
-    PartAdj pa;
-    double e0[3] = {0, 0, 0};
-    double dB1 = 0, dB2 = 0, dtp = 0, dtm = 0, dF[3] = {0, 0, 0};
+    unsigned link_ctas = 0;
+    bool graphs = false;  // long runs replay graphs, short ones launch their ticks
+    bool begun = false;
 };
 
-std::vector<std::pair<void*, size_t>> snap_regions(lbm_handle* h) {
+// what a tick reads of the model's state, and where each region lies in a stored state
+struct SnapRegion {
+    void* ptr;
+    size_t bytes, offset;
+};
+std::vector<SnapRegion> snap_regions(lbm_handle* h) {
     const size_t np = h->hparts.size();
-    return {{h->pop[h->cur], (size_t)h->N * h->q * storage_bytes(h->storage)},
-            {h->d_parts, sizeof(ParticleDev) * np},
-            {h->d_ivl, sizeof(int2) * h->ivl_slots},
-            {h->d_links, sizeof(int2) * h->link_slots},
-            {h->d_tilebits, sizeof(unsigned long long) * h->g.ntiles * h->words},
-            {h->d_nbox[0], sizeof(int) * 6 * np},
-            {h->d_nbox[1], sizeof(int) * 6 * np}};
+    std::vector<SnapRegion> v = {{h->pop[h->cur], (size_t)h->N * h->q * storage_bytes(h->storage), 0},
+                                 {h->d_parts, sizeof(ParticleDev) * np, 0},
+                                 {h->d_ivl, sizeof(int2) * h->ivl_slots, 0},
+                                 {h->d_links, sizeof(int2) * h->link_slots, 0},
+                                 {h->d_tilebits, sizeof(unsigned long long) * h->g.ntiles * h->words, 0},
+                                 {h->d_nbox[0], sizeof(int) * 6 * np, 0},
+                                 {h->d_nbox[1], sizeof(int) * 6 * np, 0}};
+    size_t at = 0;
+    for (SnapRegion& r : v) {
+        if (!r.ptr) r.bytes = 0;
+        r.offset = at;
+        at += (r.bytes + 255) / 256 * 256;
+    }
+    return v;
+}
+
+int snap_copy(AdjointRun& R, char* buf, bool save) {
+    lbm_handle* h = R.h;
+    CopyArgs c{};
+    const std::vector<SnapRegion> v = snap_regions(h);
+    static_assert(kCopyRegions == 7, "the regions above");
+    for (int k = 0; k < kCopyRegions; ++k) {
+        c.src[k] = save ? v[k].ptr : buf + v[k].offset;
+        c.dst[k] = save ? buf + v[k].offset : v[k].ptr;
+        c.bytes[k] = v[k].bytes;
+    }
+    const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>(592, c.bytes[0] / (512 * 64) + 1));
+    k_copy_regions<<<grid, 512, 0, h->stream>>>(c);
+    CUDA_TRY(h, cudaGetLastError());
+    return LBM_OK;
 }
 
 int snap_push(AdjointRun& R) {
     lbm_handle* h = R.h;
     Snap s;
-    int rc = dev_alloc(h, &s.buf, R.snap_bytes);
-    if (rc) return rc;
-    char* p = s.buf;
-    for (auto& r : snap_regions(h)) {
-        if (r.first && r.second) CUDA_TRY(h, cudaMemcpyAsync(p, r.first, r.second, cudaMemcpyDeviceToDevice, h->stream));
-        p += r.second;
+    if (!R.spare.empty()) {
+        s.buf = R.spare.back();
+        R.spare.pop_back();
+    } else {
+        const int rc = dev_alloc(h, &s.buf, R.snap_bytes);
+        if (rc) return rc;
+        R.extra.push_back(s.buf);
     }
     s.tick = h->tick;
     s.time = h->time;
     s.cur = h->cur;
     R.snaps.push_back(s);
     R.max_used = std::max(R.max_used, (int)R.snaps.size());
-    return LBM_OK;
+    return snap_copy(R, s.buf, true);
 }
 
 int snap_restore(AdjointRun& R, const Snap& s) {
@@ -3033,130 +3008,65 @@ int snap_restore(AdjointRun& R, const Snap& s) {
     h->tick = s.tick;
     h->time = s.time;
     h->part_pending = false;
-    char* p = s.buf;
-    for (auto& r : snap_regions(h)) {
-        if (r.first && r.second) CUDA_TRY(h, cudaMemcpyAsync(r.first, p, r.second, cudaMemcpyDeviceToDevice, h->stream));
-        p += r.second;
-    }
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    return LBM_OK;
+    return snap_copy(R, s.buf, false);
 }
 
 void snap_pop(AdjointRun& R) {
-    dev_free(R.snaps.back().buf);
-    R.h->device_bytes -= R.snap_bytes;
+    R.spare.push_back(R.snaps.back().buf);
     R.snaps.pop_back();
 }
 
-// k ticks forward, recording the particle after each
+// k ticks forward on the streams; the particle update writes the record after
+// each into the device history (ParticleArgs::rec), so nothing waits for them
 int advance(AdjointRun& R, long long k) {
     lbm_handle* h = R.h;
-    for (long long s = 0; s < k; ++s) {
-        int rc = lbm_step(h, 1);
+    if (R.graphs) {
+        const int rc = ensure_graphs(h, k);
         if (rc) return rc;
-        CUDA_TRY(h, cudaMemcpy(&R.rec[h->tick], h->d_parts, sizeof(ParticleDev), cudaMemcpyDeviceToHost));
-        R.have[h->tick] = 1;
-        ++R.forward;
     }
-    return LBM_OK;
+    for (long long done = 0; done < k;) {
+        int ticks = 1;
+        if (R.graphs) {
+            int g = 0;
+            while (kModelGraphSizes[g] > k - done) ++g;
+            ticks = kModelGraphSizes[g];
+            CUDA_TRY(h, cudaGraphLaunch(h->graphs[h->profiling >= 2 ? 1 : 0][h->cur][g].exec, h->stream));
+        } else {
+            enqueue_tick(h, h->cur, 0);
+        }
+        if (ticks & 1) h->cur = 1 - h->cur;
+        done += ticks;
+    }
+    join_particles(h);
+    for (long long s = 0; s < k; ++s) {
+        h->time += h->dt;
+        R.have[++h->tick] = 1;
+    }
+    R.forward += k;
+    CUDA_TRY(h, cudaGetLastError());
+    return k >= kModelGraphTicks ? check_device_error(h) : LBM_OK;  // a long segment that diverged ends the run
 }
 
-// backward step of tick n; the device holds the state at tick n and
-// rec[n + 1] is known
+// backward step of tick n; the device holds the state at tick n, and the
+// particle after tick n + 1 is in the history
 int backward_tick(AdjointRun& R, long long n) {
     lbm_handle* h = R.h;
-    const int D = h->dims;
-    const ParticleDev& P0 = R.rec[n];
-    const ParticleDev& P1 = R.rec[n + 1];
-    PartAdj& A = R.pa;
-    const double dt = h->dt;
-    // the observable reads the velocity after tick n + 1, or the force of tick n + 1
-    const bool in_window = n + 1 >= R.spec.window_begin && n + 1 <= R.spec.window_end;
-    const double K = (double)(R.spec.window_end - R.spec.window_begin + 1);
-    if (in_window && R.spec.observable == LBM_OBSERVABLE_VELOCITY)
-        for (int k = 0; k < D; ++k) A.v[k] += R.e0[k] / K;
-    // reverse the particle update of tick n (particles.cuh, moveParticles!)
-    bool moved = false, alpha = false;
-    if (P0.coupleF)
-        for (int k = 0; k < D; ++k) moved = moved || P1.v[k] != 0.0;
-    if (P0.coupleT)
-        for (int k = 0; k < (D == 2 ? 1 : 3); ++k) alpha = alpha || P1.lastT[k] * P0.inv_inertia != 0.0;
-    if (moved || alpha) {  // the snapshot after the update is the updated state
-        for (int k = 0; k < 3; ++k) {
-            A.R[k] += A.S[k];
-            A.v[k] += A.S[3 + k];
-            A.w[k] += A.S[6 + k];
-            A.e[k] += A.S[9 + k];
-        }
-        for (double& s : A.S) s = 0.0;
-    }
-    if (moved) {  // the torque arm after the update is the new position
-        for (int k = 0; k < 3; ++k) A.R[k] += A.mR[k];
-        for (double& s : A.mR) s = 0.0;
-    }
-    if (P0.coupleT && P0.kind == LBM_SQUIRMER) {  // e' = rot(e, w')
-        double le[3] = {0, 0, 0}, lw[3] = {0, 0, 0};
-        for (int q = 0; q < 6; ++q) {
-            HD e[3], w[3], o[3];
-            for (int k = 0; k < 3; ++k) {
-                e[k] = HD{P0.e[k], q == k ? 1.0 : 0.0};
-                w[k] = HD{P1.w[k], q == 3 + k ? 1.0 : 0.0};
-            }
-            rodrigues(e, w, dt, D, o);
-            double g = 0.0;
-            for (int k = 0; k < D; ++k) g += A.e[k] * o[k].d;
-            if (q < 3) le[q] = g;
-            else lw[q - 3] = g;
-        }
-        for (int k = 0; k < 3; ++k) {
-            A.e[k] = le[k];
-            A.w[k] += lw[k];
-        }
-    }
-    AdjArgs a{};
-    if (P0.coupleT)
-        for (int k = 0; k < (D == 2 ? 1 : 3); ++k) a.lamT[k] = dt * P0.inv_inertia * A.w[k];  // w' = w + dt T / I
-    if (P0.coupleF) {
-        for (int k = 0; k < D; ++k) A.v[k] += dt * A.R[k];                                    // R' = R + dt v'
-        for (int k = 0; k < D; ++k) a.lamF[k] = dt * P0.inv_mass * A.v[k];                   // v' = v + dt F / m
-    }
-    if (in_window && R.spec.observable == LBM_OBSERVABLE_FORCE)
-        for (int k = 0; k < D; ++k) a.lamF[k] += R.e0[k] / K;  // J += e.F / K
-    // the field adjoint of tick n on the device
+    AdjArgs& a = R.args;
     a.src = h->pop[h->cur];
     a.lam_in = R.lam[R.lcur];
     a.lam_out = R.lam[1 - R.lcur];
-    a.g = h->g;
-    for (int k = 0; k < 3; ++k) a.coord[k] = h->d_coord[k];
-    a.part = h->d_parts;
-    a.ivl = h->d_ivl;
-    a.wall = h->d_wall;
-    a.uw = h->d_uw;
-    a.has_part = 1;
-    a.rho0 = h->rho0;
-    a.inv_scale = 1.0 / h->scale;
-    a.dt = h->dt;
-    a.tau_p = h->tau;
-    a.tau_m = h->trt ? h->tau_minus : h->tau;
-    for (int k = 0; k < 3; ++k) a.F[k] = h->F[k];
-    a.guo = h->force_mode == LBM_FORCE_UNIFORM ? 1 : 0;
-    a.incompressible = h->incompressible;
-    a.rho_inc = h->rho_inc;
-    a.coeff = std::pow(h->dx, h->dims) / h->dt;
-    a.partial = R.partial;
-    h->ops.adjoint(a, h->stream);
-    k_adjoint_sum<kAdjAcc><<<kAdjAcc, kSumBlock, 0, h->stream>>>(R.partial, R.nblocks, R.dsum);
-    double acc[kAdjAcc];
-    CUDA_TRY(h, cudaMemcpyAsync(acc, R.dsum, sizeof(acc), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    if (!R.begun) {  // the particle update of the last tick
+        a.finish = 0;
+        a.n = n;
+        h->ops.adjoint_particle(a, h->stream);
+        R.begun = true;
+    }
+    h->ops.adjoint(a, R.link_ctas, h->stream);
+    a.finish = 1;
+    a.n = n - 1;
+    h->ops.adjoint_particle(a, h->stream);
+    CUDA_TRY(h, cudaGetLastError());
     R.lcur = 1 - R.lcur;
-    R.dtp += acc[0];
-    R.dtm += acc[1];
-    for (int k = 0; k < 3; ++k) R.dF[k] += acc[2 + k];
-    for (int k = 0; k < 12; ++k) A.S[k] += acc[5 + k];  // the snapshot tick n used
-    R.dB1 += acc[17];
-    R.dB2 += acc[18];
-    for (int k = 0; k < 3; ++k) A.mR[k] += acc[19 + k];
     return LBM_OK;
 }
 
@@ -3242,84 +3152,142 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
         return set_err(h, LBM_ERR_INVALID, "need 1 <= window_begin <= window_end <= ticks");
     if (spec->snapshots < 2) return set_err(h, LBM_ERR_INVALID, "at least two snapshots");
     if (h->tick != 0) return set_err(h, LBM_ERR_STATE, "the adjoint runs from tick 0 (a freshly built model)");
-    AdjointRun R;
-    R.h = h;
-    R.spec = *spec;
-    const long long T = spec->ticks;
-    R.rec.resize(T + 1);
-    R.have.assign(T + 1, 0);
-    R.have[0] = 1;
-    join_particles(h);
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     if (spec->observable != LBM_OBSERVABLE_VELOCITY && spec->observable != LBM_OBSERVABLE_FORCE)
         return set_err(h, LBM_ERR_INVALID, "unknown observable");
+    AdjointRun R;
+    R.h = h;
+    const long long T = spec->ticks;
+    R.have.assign(T + 1, 0);
+    R.have[0] = 1;
+    R.graphs = T >= kAdjointGraphTicks;
+    join_particles(h);
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     const int record = spec->observable == LBM_OBSERVABLE_FORCE ? 1 : 0;
     int record_before = 0;  // the caller's lbm_record_force setting, restored at the end
     CUDA_TRY(h, cudaMemcpy(&record_before, &h->d_parts[0].recordF, sizeof(int), cudaMemcpyDeviceToHost));
     // the force observable needs the momentum exchange even of a held particle
     CUDA_TRY(h, cudaMemcpy(&h->d_parts[0].recordF, &record, sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_TRY(h, cudaMemcpy(&R.rec[0], h->d_parts, sizeof(ParticleDev), cudaMemcpyDeviceToHost));
-    double en = 0.0;
+    CUDA_TRY(h, cudaMemset(&h->d_parts[0].rec_tick, 0, sizeof(int)));
+    ParticleDev P0;
+    CUDA_TRY(h, cudaMemcpy(&P0, h->d_parts, sizeof(ParticleDev), cudaMemcpyDeviceToHost));
+    double en = 0.0, e0[3];
     for (int k = 0; k < 3; ++k) en += spec->direction[k] * spec->direction[k];
-    for (int k = 0; k < 3; ++k) R.e0[k] = en > 0 ? spec->direction[k] : R.rec[0].e[k];
-    for (auto& r : snap_regions(h)) R.snap_bytes += r.second;
+    for (int k = 0; k < 3; ++k) e0[k] = en > 0 ? spec->direction[k] : P0.e[k];
+    {
+        const SnapRegion last = snap_regions(h).back();
+        R.snap_bytes = last.offset + (last.bytes + 255) / 256 * 256;
+    }
     const size_t lam_bytes = sizeof(double) * (size_t)h->N * h->q;
-    R.nblocks = (h->N + kAdjBlock - 1) / kAdjBlock;
+    const long long nblocks = (h->N + kAdjBlock - 1) / kAdjBlock;
+    R.link_ctas = (unsigned)std::min(kAdjLinkCtas, (P0.link_cap + kAdjLinkWarps - 1) / kAdjLinkWarps);
+    const size_t part_bytes = sizeof(double) * (kAdjAcc * (size_t)nblocks + kAdjLinkAcc * (size_t)R.link_ctas);
+    const size_t rec_bytes = sizeof(ParticleDev) * (size_t)(T + 1);
+    double *dmu = nullptr, *partial = nullptr;
+    AdjState* st = nullptr;
+    // the stored states in one block where it fits (a run holds up to min(snapshots, ticks + 1) of them)
+    char* arena = nullptr;
+    const size_t slots = (size_t)std::min<long long>(spec->snapshots, T + 1);
+    if (dev_alloc(h, &arena, R.snap_bytes * slots) == LBM_OK)
+        for (size_t k = slots; k-- > 0;) R.spare.push_back(arena + k * R.snap_bytes);
     int rc = dev_alloc(h, &R.lam[0], lam_bytes);
     if (!rc) rc = dev_alloc(h, &R.lam[1], lam_bytes);
-    if (!rc) rc = dev_alloc(h, &R.partial, sizeof(double) * kAdjAcc * R.nblocks);
-    if (!rc) rc = dev_alloc(h, &R.dsum, sizeof(double) * kAdjAcc);
-    if (!rc && cudaMemset(R.lam[0], 0, lam_bytes) != cudaSuccess) rc = set_err(h, LBM_ERR_CUDA, "memset failed");
+    if (!rc) rc = dev_alloc(h, &dmu, sizeof(double) * h->N);
+    if (!rc) rc = dev_alloc(h, &partial, part_bytes);
+    if (!rc) rc = dev_alloc(h, &st, sizeof(AdjState));
+    if (!rc) rc = dev_alloc(h, &h->d_rec, rec_bytes);
+    if (!rc && (cudaMemsetAsync(R.lam[0], 0, lam_bytes, h->stream) != cudaSuccess ||
+                cudaMemsetAsync(dmu, 0, sizeof(double) * h->N, h->stream) != cudaSuccess ||
+                cudaMemsetAsync(st, 0, sizeof(AdjState), h->stream) != cudaSuccess ||
+                cudaMemcpyAsync(h->d_rec, h->d_parts, sizeof(ParticleDev), cudaMemcpyDeviceToDevice, h->stream) !=
+                    cudaSuccess))
+        rc = set_err(h, LBM_ERR_CUDA, "memset failed");
+    drop_graphs(h);  // the ticks below also write the history
+    if (!rc) rc = prepare_tick(h);
+    AdjArgs& a = R.args;
+    a.dmu = dmu;
+    a.g = h->g;
+    for (int k = 0; k < 3; ++k) a.coord[k] = h->d_coord[k];
+    a.part = h->d_parts;
+    a.ivl = h->d_ivl;
+    a.links = h->d_links;
+    a.wall = h->d_wall;
+    a.uw = h->d_uw;
+    a.rho0 = h->rho0;
+    a.inv_scale = 1.0 / h->scale;
+    a.dt = h->dt;
+    a.tau_p = h->tau;
+    a.tau_m = h->trt ? h->tau_minus : h->tau;
+    for (int k = 0; k < 3; ++k) a.F[k] = h->F[k];
+    a.guo = h->force_mode == LBM_FORCE_UNIFORM ? 1 : 0;
+    a.incompressible = h->incompressible;
+    a.rho_inc = h->rho_inc;
+    a.coeff = std::pow(h->dx, h->dims) / h->dt;
+    a.st = st;
+    a.partial = partial;
+    a.lpartial = partial + kAdjAcc * nblocks;
+    a.nblocks = nblocks;
+    a.nlblocks = R.link_ctas;
+    a.rec = h->d_rec;
+    a.window_begin = spec->window_begin;
+    a.window_end = spec->window_end;
+    for (int k = 0; k < 3; ++k) a.dir[k] = e0[k];
+    a.observe_force = record;
     if (!rc) rc = snap_push(R);  // the initial state
     if (!rc) rc = reverse(R, 0, T, spec->snapshots - 1);
-    if (!rc) {  // the initial condition depends on the body force
+    AdjState G{};
+    std::vector<ParticleDev> rec;
+    if (!rc) {
         rc = snap_restore(R, R.snaps.front());
-        if (!rc && h->force_mode == LBM_FORCE_UNIFORM) {
-            AdjArgs a{};
+        if (!rc && h->force_mode == LBM_FORCE_UNIFORM) {  // the initial condition depends on the body force
             a.src = h->pop[h->cur];
             a.lam_in = R.lam[R.lcur];
-            a.g = h->g;
-            a.rho0 = h->rho0;
-            a.inv_scale = 1.0 / h->scale;
-            a.dt = h->dt;
-            a.guo = 1;
-            a.incompressible = h->incompressible;
-            a.rho_inc = h->rho_inc;
-            a.partial = R.partial;
             h->ops.adjoint_init(a, h->stream);
-            k_adjoint_sum<kAdjAcc><<<kAdjAcc, kSumBlock, 0, h->stream>>>(R.partial, R.nblocks, R.dsum);
-            double acc[kAdjAcc];
+            if (cudaMemsetAsync(a.lpartial, 0, sizeof(double) * kAdjLinkAcc * R.link_ctas, h->stream) != cudaSuccess)
+                rc = set_err(h, LBM_ERR_CUDA, "memset failed");
+            a.finish = 1;
+            a.n = -1;
+            h->ops.adjoint_particle(a, h->stream);
+        }
+        if (!rc) {
+            rec.resize(T + 1);
             // on the handle's stream: a plain cudaMemcpy would not wait for it
-            if (cudaMemcpyAsync(acc, R.dsum, sizeof(acc), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
+            if (cudaMemcpyAsync(&G, st, sizeof(G), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
+                cudaMemcpyAsync(rec.data(), h->d_rec, rec_bytes, cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
                 cudaStreamSynchronize(h->stream) != cudaSuccess)
                 rc = set_err(h, LBM_ERR_CUDA, "read-back failed");
             else
-                for (int k = 0; k < 3; ++k) R.dF[k] += acc[k];
+                rc = check_device_error(h);
         }
     }
-    while (!R.snaps.empty()) snap_pop(R);
+    cudaStreamSynchronize(h->stream);  // nothing below is in use any more, after an error either
+    h->device_bytes -= R.snap_bytes * (R.extra.size() + (arena ? slots : 0));
+    dev_free(arena);
+    for (char*& s : R.extra) dev_free(s);
     if (cudaMemcpy(&h->d_parts[0].recordF, &record_before, sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess &&
         !rc)
         rc = set_err(h, LBM_ERR_CUDA, "cannot restore the force record flag");
     dev_free(R.lam[0]);
     dev_free(R.lam[1]);
-    dev_free(R.partial);
-    dev_free(R.dsum);
-    h->device_bytes -= 2 * lam_bytes + sizeof(double) * kAdjAcc * (R.nblocks + 1);
+    dev_free(dmu);
+    dev_free(partial);
+    dev_free(st);
+    dev_free(h->d_rec);
+    drop_graphs(h);  // they write the history
+    h->device_bytes -= 2 * lam_bytes + sizeof(double) * h->N + part_bytes + sizeof(AdjState) +
+                       rec_bytes;
     if (rc) return rc;
     std::memset(out, 0, sizeof(*out));
     const double K = (double)(spec->window_end - spec->window_begin + 1);
     double J = 0.0;
     for (long long t = spec->window_begin; t <= spec->window_end; ++t)
-        for (int k = 0; k < h->dims; ++k)
-            J += (record ? R.rec[t].lastF[k] : R.rec[t].v[k]) * R.e0[k] / K;
+        for (int k = 0; k < h->dims; ++k) J += (record ? rec[t].lastF[k] : rec[t].v[k]) * e0[k] / K;
     out->value = J;
-    out->dB1 = R.dB1;
-    out->dB2 = R.dB2;
-    out->dtau_plus = R.dtp;
-    out->dtau_minus = h->trt ? R.dtm : 0.0;
-    out->dtau = R.dtp + (h->trt ? spec->tau_minus_slope * R.dtm : 0.0);
-    for (int k = 0; k < 3; ++k) out->dF[k] = k < h->dims ? R.dF[k] : 0.0;
+    out->dB1 = G.dB1;
+    out->dB2 = G.dB2;
+    out->dtau_plus = G.dtp;
+    out->dtau_minus = h->trt ? G.dtm : 0.0;
+    out->dtau = G.dtp + (h->trt ? spec->tau_minus_slope * G.dtm : 0.0);
+    for (int k = 0; k < 3; ++k) out->dF[k] = k < h->dims ? G.dF[k] : 0.0;
     out->forward_ticks = R.forward;
     out->snapshots_used = R.max_used;
     out->ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

@@ -40,7 +40,8 @@ struct Ops {
     // a batch's bulk tiles, one CTA per entry of dmap
     void (*bulk_batch)(const StepArgs* args, const int2* dmap, long long tiles, cudaStream_t, bool sr, bool reverse);
     // discrete adjoint of one tick, and of the initial condition (adjoint.cuh)
-    void (*adjoint)(const AdjArgs&, cudaStream_t);
+    void (*adjoint)(const AdjArgs&, unsigned link_ctas, cudaStream_t);  // link terms, then the nodes
+    void (*adjoint_particle)(const AdjArgs&, cudaStream_t);
     void (*adjoint_init)(const AdjArgs&, cudaStream_t);
     const void* bulk_fn;      // kernel symbols (occupancy queries, attributes)
     const void* bulk_tma_fn;
@@ -131,8 +132,12 @@ struct OpsImpl {
             k_bulk_batch<L, ST, TRT, false><<<(unsigned)tiles, kTickBlock, 0, s>>>(args, dmap, reverse ? 1 : 0);
         }
     }
-    static void adjoint(const AdjArgs& a, cudaStream_t s) {
+    static void adjoint(const AdjArgs& a, unsigned link_ctas, cudaStream_t s) {
+        k_adjoint_links<L, ST, TRT><<<link_ctas, 32 * kAdjLinkWarps, 0, s>>>(a);
         k_adjoint<L, ST, TRT><<<blocks_for(a.g.N, kAdjBlock), kAdjBlock, 0, s>>>(a);
+    }
+    static void adjoint_particle(const AdjArgs& a, cudaStream_t s) {
+        k_adjoint_particle<L::D><<<1, kAdjSumBlock, 0, s>>>(a);
     }
     static void adjoint_init(const AdjArgs& a, cudaStream_t s) {
         k_adjoint_init<L, ST><<<blocks_for(a.g.N, kAdjBlock), kAdjBlock, 0, s>>>(a);
@@ -171,6 +176,7 @@ struct OpsImpl {
         o.tick = ST == ST_F64 ? nullptr : tick;
         o.bulk_batch = ST == ST_F64 ? nullptr : bulk_batch;
         o.adjoint = adjoint;
+        o.adjoint_particle = adjoint_particle;
         o.adjoint_init = adjoint_init;
         o.bulk_fn = (const void*)k_bulk<L, ST, TRT>;
         o.fixup_fn = (const void*)k_fixup<L, ST, TRT>;

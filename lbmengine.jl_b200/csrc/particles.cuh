@@ -44,8 +44,22 @@ struct ParticleArgs {
     double* trj;       // trajectory ring: [trj_cap][nparts][9] (position, velocity, angular
                        // velocity after each tick's update), or null
     long long trj_cap;
+    ParticleDev* rec;    // the particle's record after each tick, [ticks + 1] (one particle), or null
     const double* fint;  // [nparts][3] forces of the particle interactions (interactions.cuh), or null
 };
+
+// the updated record P (in shared memory) back to global memory, and into the
+// history lbm_adjoint keeps; every thread of the CTA, after a barrier
+__device__ __forceinline__ void store_record(const ParticleArgs& a, int p, const ParticleDev& P) {
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&P);
+    unsigned long long* dst = reinterpret_cast<unsigned long long*>(a.parts + p);
+    unsigned long long* rec =
+        a.rec && a.mode == 0 ? reinterpret_cast<unsigned long long*>(a.rec + P.rec_tick) : nullptr;
+    for (int k = threadIdx.x; k < (int)(sizeof(ParticleDev) / 8); k += blockDim.x) {
+        dst[k] = src[k];
+        if (rec) rec[k] = src[k];
+    }
+}
 
 // publish particle p's solid box for the far/near split of the bulk pass
 __device__ __forceinline__ void publish_box(const ParticleArgs& a, int p, const ParticleDev& P) {
@@ -219,6 +233,7 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
     }
     __syncthreads();
     ParticleDev& P = sP;
+    if (tid == 0 && a.rec && a.mode == 0) P.rec_tick += 1;
     if (tid == 0) P.relink = 0;  // set again below when this update changes the intervals
 
     // 1. momentum exchange: fixed-order reduction of the per-chunk partials
@@ -419,9 +434,7 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
     __syncthreads();
     if (!s_moved || s_keep) {
         // nothing geometric changed; write the record back
-        const unsigned long long* ssrc = reinterpret_cast<const unsigned long long*>(&sP);
-        unsigned long long* gdst = reinterpret_cast<unsigned long long*>(a.parts + p);
-        for (int k = tid; k < (int)(sizeof(ParticleDev) / 8); k += blockDim.x) gdst[k] = ssrc[k];
+        store_record(a, p, P);
         if (tid == 0) publish_box(a, p, P);
         return;
     }
@@ -635,12 +648,8 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
         for (int r = tid; r < s_rows; r += blockDim.x) a.ivl[P.ivl_off + r] = s_ivl[r];
     if (s_changed && a.inline_links)
         for (int e = tid; e < s_lkn; e += blockDim.x) a.links[P.link_off + e] = s_lk[e];
-    {
-        const unsigned long long* ssrc = reinterpret_cast<const unsigned long long*>(&sP);
-        unsigned long long* gdst = reinterpret_cast<unsigned long long*>(a.parts + p);
-        for (int k = tid; k < (int)(sizeof(ParticleDev) / 8); k += blockDim.x) gdst[k] = ssrc[k];
-        if (tid == 0) publish_box(a, p, P);
-    }
+    store_record(a, p, P);
+    if (tid == 0) publish_box(a, p, P);
 }
 
 template <class L>
