@@ -540,7 +540,7 @@ int lbm_step_noalloc(lbm_handle* h, int64_t nsteps);
 
 /* lbm_destroy waits for the handle's queued work and gives its device
  * buffers back.  The library keeps freed device blocks (up to 4 GiB in the
- * process) for later allocations of the same size, so a model built after
+ * process, the ones freed longest ago giving way) for later allocations of the same size, so a model built after
  * another does not pay cudaMalloc again; the kept blocks go back to the
  * driver when a cudaMalloc fails. */
 const char* lbm_last_error(lbm_handle* h);

@@ -53,6 +53,11 @@ constexpr int kModelGraphTicks = kModelGraphSizes[0];
 // Later calls build and replay graphs.
 constexpr int kFirstCallDirectTicks = 32;
 static_assert(kFirstCallDirectTicks <= kModelGraphTicks, "profiling slots");
+// lbm_get_fields into pinned memory: fields of up to this many bytes (64^2: 28 -> 22 us a
+// read, 256^2 54 -> 49, 512^2 no difference) are
+// written by the kernel over the host link, without device scratch or copies;
+// larger ones go through the copy engine.
+constexpr size_t kMappedReadBytes = size_t(4) << 20;
 // lbm_adjoint runs of at least this many ticks build graphs for their forward
 // ticks (one to a few recomputations of every tick repay the build), shorter
 // ones launch them directly.
@@ -199,13 +204,22 @@ std::atomic<long long> g_mem_limit{0};
 // short run) does not pay for them again.  A stream-ordered memory pool gave
 // the same saving, but the bulk pass ran 1-1.5 % slower on its memory.  A
 // freed block is kept only after its device has finished its queued work,
-// as cudaFree waits for it.
+// as cudaFree waits for it.  Where the kept blocks would exceed kKeepBytes, the
+// ones freed longest ago go back to the driver: a process that moves from
+// large models to small ones otherwise keeps blocks that nothing asks for and
+// pays cudaMalloc and cudaFree for every buffer of the small ones.
 constexpr size_t kKeepBytes = size_t(4) << 30;
 struct BlockCache {
     std::mutex mu;
-    std::multimap<size_t, std::pair<int, void*>> kept;        // capacity -> (device, block)
+    struct Kept {
+        int dev;
+        void* p;
+        unsigned long long freed;  // order of the frees
+    };
+    std::multimap<size_t, Kept> kept;                        // capacity -> block
     std::unordered_map<void*, std::pair<int, size_t>> live;  // block -> (device, capacity)
     size_t kept_bytes = 0;
+    unsigned long long frees = 0;
 };
 BlockCache g_blocks;
 
@@ -215,8 +229,8 @@ void release_kept(int dev) {
     {
         std::lock_guard<std::mutex> lk(g_blocks.mu);
         for (auto it = g_blocks.kept.begin(); it != g_blocks.kept.end();) {
-            if (it->second.first == dev) {
-                drop.push_back(it->second.second);
+            if (it->second.dev == dev) {
+                drop.push_back(it->second.p);
                 g_blocks.kept_bytes -= it->first;
                 it = g_blocks.kept.erase(it);
             } else {
@@ -238,8 +252,8 @@ cudaError_t block_alloc(void** p, size_t bytes) {
         std::lock_guard<std::mutex> lk(g_blocks.mu);
         for (auto it = g_blocks.kept.lower_bound(bytes);
              it != g_blocks.kept.end() && it->first <= bytes + bytes / 8; ++it) {
-            if (it->second.first != dev) continue;
-            *p = it->second.second;
+            if (it->second.dev != dev) continue;
+            *p = it->second.p;
             g_blocks.live[*p] = {dev, it->first};
             g_blocks.kept_bytes -= it->first;
             g_blocks.kept.erase(it);
@@ -259,7 +273,8 @@ cudaError_t block_alloc(void** p, size_t bytes) {
     return e;
 }
 
-// give back a block from block_alloc: kept when there is room, else cudaFree
+// give back a block from block_alloc: kept, in place of the blocks freed
+// longest ago where room is short; cudaFree for one larger than kKeepBytes
 void block_free(void* p) {
     int dev = -1;
     size_t cap = 0;
@@ -279,20 +294,29 @@ void block_free(void* p) {
     int cur = 0;
     cudaGetDevice(&cur);
     if (dev != cur) cudaSetDevice(dev);
-    bool kept = false;
-    if (cudaDeviceSynchronize() == cudaSuccess) {
+    std::vector<std::pair<int, void*>> drop;
+    if (cap <= kKeepBytes && cudaDeviceSynchronize() == cudaSuccess) {
         std::lock_guard<std::mutex> lk(g_blocks.mu);
-        if (g_blocks.kept_bytes + cap <= kKeepBytes) {
-            g_blocks.kept.emplace(cap, std::make_pair(dev, p));
-            g_blocks.kept_bytes += cap;
-            kept = true;
+        while (g_blocks.kept_bytes + cap > kKeepBytes) {
+            auto old = g_blocks.kept.begin();
+            for (auto it = g_blocks.kept.begin(); it != g_blocks.kept.end(); ++it)
+                if (it->second.freed < old->second.freed) old = it;
+            drop.push_back({old->second.dev, old->second.p});
+            g_blocks.kept_bytes -= old->first;
+            g_blocks.kept.erase(old);
         }
-    }
-    if (!kept) {
+        g_blocks.kept.emplace(cap, BlockCache::Kept{dev, p, g_blocks.frees++});
+        g_blocks.kept_bytes += cap;
+    } else {
         cudaGetLastError();
-        cudaFree(p);
+        drop.push_back({dev, p});
     }
-    if (dev != cur) cudaSetDevice(cur);
+    for (auto& d : drop) {
+        cudaSetDevice(d.first);
+        cudaFree(d.second);
+    }
+    int now = 0;
+    if (cudaGetDevice(&now) != cudaSuccess || now != cur) cudaSetDevice(cur);
 }
 
 template <class P>
@@ -319,6 +343,76 @@ template <class P>
 void dev_free(P*& p) {
     if (p) block_free((void*)p);
     p = nullptr;
+}
+
+// Pinned host memory for small read-backs (error words, particle records), in
+// chunks that outlive their user: a copy to pageable memory is staged by the
+// driver, which waits for the stream and takes several microseconds more per
+// call.  A lease holds one chunk for one call, so threads never share one; at
+// most as many chunks exist as calls ran at once.
+constexpr size_t kPinnedChunk = 192 * 1024;  // 255 particle records
+struct PinnedChunks {
+    std::mutex mu;
+    std::vector<void*> free;
+};
+PinnedChunks g_pinned;
+struct PinnedLease {
+    void* p = nullptr;
+    explicit PinnedLease(size_t bytes) {
+        if (bytes > kPinnedChunk) return;  // the caller copies to pageable memory
+        {
+            std::lock_guard<std::mutex> lk(g_pinned.mu);
+            if (!g_pinned.free.empty()) {
+                p = g_pinned.free.back();
+                g_pinned.free.pop_back();
+                return;
+            }
+        }
+        if (cudaHostAlloc(&p, kPinnedChunk, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+    }
+    ~PinnedLease() {
+        if (!p) return;
+        std::lock_guard<std::mutex> lk(g_pinned.mu);
+        g_pinned.free.push_back(p);
+    }
+    PinnedLease(const PinnedLease&) = delete;
+    PinnedLease& operator=(const PinnedLease&) = delete;
+};
+
+// copy `bytes` from the device through a pinned chunk into `dst`, after the
+// stream's queued work
+cudaError_t read_small(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    PinnedLease l(bytes);
+    cudaError_t e = cudaMemcpyAsync(l.p ? l.p : dst, src, bytes, cudaMemcpyDeviceToHost, s);
+    const cudaError_t e2 = cudaStreamSynchronize(s);  // also after an error: the chunk goes back to the pool
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess && l.p) std::memcpy(dst, l.p, bytes);
+    return e;
+}
+
+// The device's address of the caller's array where a kernel can write it in
+// place: pinned host memory (cudaHostAlloc, cudaHostRegister) mapped for the
+// current device, from its first to its last byte; else null.
+double* mapped_host(double* host, size_t bytes) {
+    if (!host || !bytes) return nullptr;
+    void* dev[2] = {nullptr, nullptr};
+    const char* at[2] = {reinterpret_cast<char*>(host), reinterpret_cast<char*>(host) + bytes - 1};
+    for (int k = 0; k < 2; ++k) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, at[k]) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+        dev[k] = a.devicePointer;
+    }
+    return static_cast<char*>(dev[1]) - static_cast<char*>(dev[0]) == (long long)bytes - 1 &&
+                   reinterpret_cast<size_t>(dev[0]) % sizeof(double) == 0
+               ? static_cast<double*>(dev[0])
+               : nullptr;
 }
 
 bool get_ops(int lattice, int storage, int trt, Ops* o) {
@@ -869,8 +963,7 @@ int ensure_graphs(lbm_handle* h, int64_t nsteps) {
 // (lbm_load_state) or destroy the handle.
 int check_device_error(lbm_handle* h) {
     int err = 0;
-    CUDA_TRY(h, cudaMemcpyAsync(&err, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    CUDA_TRY(h, read_small(&err, h->d_err, sizeof(int), h->stream));
     if (err == 0) return LBM_OK;
     CUDA_TRY(h, cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -1794,12 +1887,25 @@ int lbm_time_kernel(lbm_handle* h, int32_t kernel, int32_t launches, double* avg
 int lbm_get_fields(lbm_handle* h, double* rho, double* u) {
     if (!h) return set_err(h, LBM_ERR_INVALID, "null handle");
     BIND(h);
-    const size_t nb = sizeof(double) * h->N * (1 + h->dims);
-    int rc = ensure_tmp(h, nb);
-    if (rc) return rc;
+    const size_t rb = sizeof(double) * h->N, ub = rb * h->dims;
     CodecArgs c = codec_args(h);
-    c.rho = h->d_tmp;
-    c.u = h->d_tmp + h->N;
+    // small fields that go to pinned memory: the kernel writes them there itself
+    if (rb + ub <= kMappedReadBytes) {
+        c.rho = mapped_host(rho, rb);
+        c.u = mapped_host(u, ub);
+    }
+    if ((rho && !c.rho) || (u && !c.u)) {
+        int rc = ensure_tmp(h, rb + ub);
+        if (rc) return rc;
+        c.rho = h->d_tmp;
+        c.u = h->d_tmp + h->N;
+    } else {
+        if (!rho && !u) return LBM_OK;
+        h->ops.macro(c, h->stream);
+        CUDA_TRY(h, cudaGetLastError());
+        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+        return LBM_OK;
+    }
     h->ops.macro(c, h->stream);
     CUDA_TRY(h, cudaGetLastError());
     if (rho) CUDA_TRY(h, cudaMemcpyAsync(rho, c.rho, sizeof(double) * h->N, cudaMemcpyDeviceToHost, h->stream));
@@ -1999,8 +2105,7 @@ int lbm_get_particles(lbm_handle* h, lbm_particle_state* out, int32_t capacity, 
     if (count) *count = np;
     if (!out || capacity <= 0 || np == 0) return LBM_OK;
     std::vector<ParticleDev> tmp(np);
-    CUDA_TRY(h, cudaMemcpyAsync(tmp.data(), h->d_parts, sizeof(ParticleDev) * np, cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    CUDA_TRY(h, read_small(tmp.data(), h->d_parts, sizeof(ParticleDev) * np, h->stream));
     for (int i = 0; i < np && i < capacity; ++i) {
         const ParticleDev& P = tmp[i];
         lbm_particle_state& s = out[i];
@@ -2560,8 +2665,7 @@ int batch_graph(lbm_batch* b, int s0) {
 int batch_check(lbm_batch* b) {
     const size_t n = b->reps.size();
     std::vector<int> err(n + 1, 0);
-    BCUDA_TRY(b, cudaMemcpyAsync(err.data(), b->d_err, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, b->stream));
-    BCUDA_TRY(b, cudaStreamSynchronize(b->stream));
+    BCUDA_TRY(b, read_small(err.data(), b->d_err, sizeof(int) * (n + 1), b->stream));
     bool any = false;
     for (size_t r = 0; r <= n; ++r) any = any || err[r] != 0;
     if (any) {  // reported below; the words start from zero again

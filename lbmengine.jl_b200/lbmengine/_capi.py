@@ -198,7 +198,7 @@ PROTOTYPES = [
     ("lbm_create", C.c_int, [C.POINTER(LbmConfig), C.POINTER(C.c_void_p)]),
     ("lbm_add_particle", C.c_int, [C.c_void_p, C.POINTER(LbmParticleParams), C.POINTER(C.c_int32)]),
     ("lbm_step", C.c_int, [C.c_void_p, C.c_int64]),
-    ("lbm_get_fields", C.c_int, [C.c_void_p, _dp, _dp]),
+    ("lbm_get_fields", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
     ("lbm_get_distributions", C.c_int, [C.c_void_p, _dp]),
     ("lbm_get_stress", C.c_int, [C.c_void_p, _dp]),
     ("lbm_get_totals", C.c_int, [C.c_void_p, _dp, _dp]),

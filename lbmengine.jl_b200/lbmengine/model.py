@@ -97,8 +97,8 @@ class LBMmodel:
             if a is not None and (a.dtype != np.float64 or a.shape != shape or not a.flags.f_contiguous
                                   or not a.flags.writeable):
                 raise ValueError(f"expected a writeable column-major float64 array of shape {shape}")
-        self._check(self._lib.lbm_get_fields(self._h, None if rho is None else rho.ctypes.data_as(capi._dp),
-                                             None if u is None else u.ctypes.data_as(capi._dp)))
+        self._check(self._lib.lbm_get_fields(self._h, None if rho is None else rho.ctypes.data,
+                                             None if u is None else u.ctypes.data))
 
     @property
     def massDensity(self) -> np.ndarray:
