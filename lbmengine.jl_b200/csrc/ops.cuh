@@ -7,6 +7,7 @@
 #include "particles.cuh"
 #include "aux_kernels.cuh"
 #include "tick.cuh"
+#include "resident.cuh"
 #include "adjoint.cuh"
 
 namespace lbm {
@@ -39,6 +40,12 @@ struct Ops {
                  int* err, unsigned grid, cudaStream_t, bool sr);
     // a batch's bulk tiles, one CTA per entry of dmap
     void (*bulk_batch)(const StepArgs* args, const int2* dmap, long long tiles, cudaStream_t, bool sr, bool reverse);
+    // many ticks of a small model in one launch (resident.cuh), null where it is not built: clusters of
+    // `csize` CTAs, or (csize 0) one cooperative grid of `ctas`
+    cudaError_t (*resident)(const ResidentArgs&, int ctas, int csize, cudaStream_t);
+    void (*resident_wmask)(const unsigned char* wall, const GridDesc&, unsigned* wmask, cudaStream_t);
+    const void* resident_fn;
+    size_t (*resident_smem)(int max_entries);  // dynamic shared memory per CTA
     // discrete adjoint of one tick, and of the initial condition (adjoint.cuh)
     void (*adjoint)(const AdjArgs&, unsigned link_ctas, cudaStream_t);  // link terms, then the nodes
     void (*adjoint_particle)(const AdjArgs&, cudaStream_t);
@@ -132,6 +139,36 @@ struct OpsImpl {
             k_bulk_batch<L, ST, TRT, false><<<(unsigned)tiles, kTickBlock, 0, s>>>(args, dmap, reverse ? 1 : 0);
         }
     }
+    static constexpr bool kResident = L::D == 2 && (ST == ST_F32 || ST == ST_F64);
+    static size_t resident_smem(int entries) {
+        if constexpr (kResident) return ResidentBoundary<L, ST>::bytes(entries);
+        return 0;
+    }
+    static void resident_wmask(const unsigned char* wall, const GridDesc& g, unsigned* wmask, cudaStream_t s) {
+        k_resident_wmask<L><<<blocks_for(g.N, 256), 256, 0, s>>>(wall, g, wmask);
+    }
+    static cudaError_t resident(const ResidentArgs& a, int ctas, int csize, cudaStream_t s) {
+        if constexpr (kResident) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)ctas);
+            cfg.blockDim = dim3(kResThreads);
+            cfg.dynamicSmemBytes = resident_smem(a.max_entries);
+            cfg.stream = s;
+            cudaLaunchAttribute attr[1];
+            if (csize > 0) {
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = (unsigned)csize;
+                attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            } else {  // the grid barrier needs every CTA resident
+                attr[0].id = cudaLaunchAttributeCooperative;
+                attr[0].val.cooperative = 1;
+            }
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            return cudaLaunchKernelEx(&cfg, k_resident<L, ST, TRT>, a);
+        }
+        return cudaErrorNotSupported;
+    }
     static void adjoint(const AdjArgs& a, unsigned link_ctas, cudaStream_t s) {
         k_adjoint_links<L, ST, TRT><<<link_ctas, 32 * kAdjLinkWarps, 0, s>>>(a);
         k_adjoint<L, ST, TRT><<<blocks_for(a.g.N, kAdjBlock), kAdjBlock, 0, s>>>(a);
@@ -175,6 +212,11 @@ struct OpsImpl {
         }
         o.tick = ST == ST_F64 ? nullptr : tick;
         o.bulk_batch = ST == ST_F64 ? nullptr : bulk_batch;
+        o.resident = kResident ? resident : nullptr;
+        o.resident_wmask = resident_wmask;
+        o.resident_smem = resident_smem;
+        o.resident_fn = nullptr;
+        if constexpr (kResident) o.resident_fn = (const void*)k_resident<L, ST, TRT>;
         o.adjoint = adjoint;
         o.adjoint_particle = adjoint_particle;
         o.adjoint_init = adjoint_init;

@@ -127,6 +127,34 @@ __device__ __forceinline__ void tile_bits_update(const ParticleArgs& a, const in
     }
 }
 
+// Rodrigues' rotation of the swimming direction e by |w| dt about w, normalised
+// (moveParticles!, src/gpu/particles.jl:48-70); 2D: w[0] about the z axis
+template <int D>
+__device__ __forceinline__ void rotate_direction(const double* w, double dt, double* e) {
+    double theta = D == 2 ? fabs(w[0]) : sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+    if (theta == 0.0) return;
+    const double* v = e;
+    double vr[3] = {0, 0, 0}, ct, st;
+    if (D == 2) {
+        const double k = w[0] / theta;
+        theta *= dt;
+        sincos(theta, &st, &ct);
+        vr[0] = v[0] * ct + (-k * v[1]) * st;
+        vr[1] = v[1] * ct + (k * v[0]) * st;
+    } else {
+        const double k[3] = {w[0] / theta, w[1] / theta, w[2] / theta};
+        theta *= dt;
+        sincos(theta, &st, &ct);
+        const double cr[3] = {k[1] * v[2] - k[2] * v[1], -k[0] * v[2] + k[2] * v[0], k[0] * v[1] - k[1] * v[0]};
+        const double kv = k[0] * v[0] + k[1] * v[1] + k[2] * v[2];
+        for (int q = 0; q < 3; ++q) vr[q] = v[q] * ct + cr[q] * st + k[q] * kv * (1.0 - ct);
+    }
+    double nr = 0.0;
+    for (int q = 0; q < D; ++q) nr += vr[q] * vr[q];
+    nr = sqrt(nr);
+    for (int q = 0; q < D; ++q) e[q] = vr[q] / nr;
+}
+
 // interval of row (y, z) of P's solid box (rows y-fastest from `rows`), or empty
 __device__ __forceinline__ int2 box_row_ivl(const ParticleDev& P, const int2* rows, int y, int z) {
     if (y < P.slo[1] || y > P.shi[1] || z < P.slo[2] || z > P.shi[2]) return make_int2(1, 0);
@@ -202,11 +230,15 @@ __device__ __forceinline__ int near_row_links(const ParticleDev& P, const int2* 
     return cnt;
 }
 
+// The update of particle p, whose record P lies in shared memory and is
+// written back by the caller; every thread of the CTA, after a barrier.
+// Returns whether the solid region was looked at again (the same value in
+// every thread): false when the stored intervals were kept.
 // LK: link entries staged in shared memory during a rebuild (kLinkSmem for
-// the particle kernel; less inside the persistent tick kernel, whose CTAs
-// also hold the bulk and fix-up items' shared memory)
+// the particle kernel; less inside the persistent kernels, whose CTAs also
+// hold the shared memory of their other work)
 template <class L, int LK = kLinkSmem>
-__device__ __forceinline__ void particles_body(const ParticleArgs& a, const int p) {
+__device__ __forceinline__ bool particles_core(const ParticleArgs& a, const int p, ParticleDev& P) {
     constexpr int D = L::D;
     const int tid = threadIdx.x;
     __shared__ double s_red[kMaxPartWarps][6];
@@ -222,17 +254,6 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
     // queued behind them.
     __shared__ int2 s_lk[LK];
     __shared__ int s_lkn;  // entries [0, s_lkn) of the new list are in s_lk
-    // the particle record is staged in shared memory: the update below is a
-    // serial chain of reads and writes that must not go to global memory
-    __shared__ ParticleDev sP;
-    static_assert(sizeof(ParticleDev) % 8 == 0, "ParticleDev is copied in 8-byte words");
-    {
-        const unsigned long long* gsrc = reinterpret_cast<const unsigned long long*>(a.parts + p);
-        unsigned long long* sdst = reinterpret_cast<unsigned long long*>(&sP);
-        for (int k = tid; k < (int)(sizeof(ParticleDev) / 8); k += blockDim.x) sdst[k] = gsrc[k];
-    }
-    __syncthreads();
-    ParticleDev& P = sP;
     if (tid == 0 && a.rec && a.mode == 0) P.rec_tick += 1;
     if (tid == 0) P.relink = 0;  // set again below when this update changes the intervals
 
@@ -311,32 +332,7 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
                 double Al[3] = {0, 0, 0};
                 for (int k = 0; k < nw2; ++k) Al[k] = T[k] * P.inv_inertia;
                 for (int k = 0; k < nw2; ++k) P.w[k] = P.w[k] + dt * Al[k];
-                if (P.kind == 1) {
-                    double theta = D == 2 ? fabs(P.w[0]) : sqrt(P.w[0] * P.w[0] + P.w[1] * P.w[1] + P.w[2] * P.w[2]);
-                    if (theta != 0.0) {  // Rodrigues' rotation of the swimming direction
-                        const double* v = P.e;
-                        double vr[3] = {0, 0, 0};
-                        if (D == 2) {
-                            const double k = P.w[0] / theta;
-                            theta *= dt;
-                            const double ct = cos(theta), st = sin(theta);
-                            vr[0] = v[0] * ct + (-k * v[1]) * st;
-                            vr[1] = v[1] * ct + (k * v[0]) * st;
-                        } else {
-                            const double k[3] = {P.w[0] / theta, P.w[1] / theta, P.w[2] / theta};
-                            theta *= dt;
-                            const double ct = cos(theta), st = sin(theta);
-                            const double cr[3] = {k[1] * v[2] - k[2] * v[1], -k[0] * v[2] + k[2] * v[0],
-                                                  k[0] * v[1] - k[1] * v[0]};
-                            const double kv = k[0] * v[0] + k[1] * v[1] + k[2] * v[2];
-                            for (int q = 0; q < 3; ++q) vr[q] = v[q] * ct + cr[q] * st + k[q] * kv * (1.0 - ct);
-                        }
-                        double nr = 0.0;
-                        for (int q = 0; q < D; ++q) nr += vr[q] * vr[q];
-                        nr = sqrt(nr);
-                        for (int q = 0; q < D; ++q) P.e[q] = vr[q] / nr;
-                    }
-                }
+                if (P.kind == 1) rotate_direction<D>(P.w, dt, P.e);
                 for (int k = 0; k < nw2; ++k)
                     if (Al[k] != 0.0) alpha = true;
             }
@@ -433,10 +429,7 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
     }
     __syncthreads();
     if (!s_moved || s_keep) {
-        // nothing geometric changed; write the record back
-        store_record(a, p, P);
-        if (tid == 0) publish_box(a, p, P);
-        return;
+        return false;  // nothing geometric changed
     }
 
     // 3. solid intervals of the new position, compared with the stored ones
@@ -648,8 +641,22 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
         for (int r = tid; r < s_rows; r += blockDim.x) a.ivl[P.ivl_off + r] = s_ivl[r];
     if (s_changed && a.inline_links)
         for (int e = tid; e < s_lkn; e += blockDim.x) a.links[P.link_off + e] = s_lk[e];
-    store_record(a, p, P);
-    if (tid == 0) publish_box(a, p, P);
+    return true;
+}
+
+template <class L, int LK = kLinkSmem>
+__device__ __forceinline__ void particles_body(const ParticleArgs& a, const int p) {
+    // the particle record is staged in shared memory: the update is a serial
+    // chain of reads and writes that must not go to global memory
+    __shared__ ParticleDev sP;
+    static_assert(sizeof(ParticleDev) % 8 == 0, "ParticleDev is copied in 8-byte words");
+    const unsigned long long* gsrc = reinterpret_cast<const unsigned long long*>(a.parts + p);
+    unsigned long long* sdst = reinterpret_cast<unsigned long long*>(&sP);
+    for (int k = threadIdx.x; k < (int)(sizeof(ParticleDev) / 8); k += blockDim.x) sdst[k] = gsrc[k];
+    __syncthreads();
+    particles_core<L, LK>(a, p, sP);
+    store_record(a, p, sP);
+    if (threadIdx.x == 0) publish_box(a, p, sP);
 }
 
 template <class L>
