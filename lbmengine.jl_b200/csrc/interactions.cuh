@@ -62,15 +62,12 @@ __device__ __forceinline__ void icross_scalar(double w, const double* v, double*
     out[2] = 0.0;
 }
 
-__device__ void interaction_forces(const InterArgs& a, int t) {
-    const InterItem it = a.items[t];
-    const int d = a.dims;
-    double* out = a.pf + (size_t)t * 9;
+// the forces of one item: on id1 (out[0..2]), and for bond angles on id3
+// (out[3..5]) and, subtracted, on id2 (out[6..8])
+__device__ __forceinline__ void interaction_force(const InterItem& it, int d, const double* R1, const double* R2,
+                                                  const double* R3, double* out) {
     for (int k = 0; k < 9; ++k) out[k] = 0.0;
-    const double* R1 = a.parts[it.id1].R;
-    const double* R2 = a.parts[it.id2].R;
     if (it.kind == 2) {  // applyInteraction!(::PolarInteraction), particles.jl:140-162
-        const double* R3 = a.parts[it.id3].R;
         double d12[3] = {0, 0, 0}, d32[3] = {0, 0, 0}, u12[3] = {0, 0, 0}, u32[3] = {0, 0, 0};
         for (int k = 0; k < d; ++k) {
             d12[k] = R1[k] - R2[k];
@@ -145,7 +142,13 @@ __device__ void interaction_forces(const InterArgs& a, int t) {
     for (int k = 0; k < d; ++k) out[k] = f * u[k];
 }
 
-__global__ void __launch_bounds__(kInterThreads) k_interactions(const InterArgs a) {
+static __device__ __forceinline__ void interaction_forces(const InterArgs& a, int t) {
+    const InterItem it = a.items[t];
+    interaction_force(it, a.dims, a.parts[it.id1].R, a.parts[it.id2].R, it.kind == 2 ? a.parts[it.id3].R : nullptr,
+                      a.pf + (size_t)t * 9);
+}
+
+static __global__ void __launch_bounds__(kInterThreads) k_interactions(const InterArgs a) {
     for (int t = threadIdx.x; t < a.nitems; t += blockDim.x) interaction_forces(a, t);
     __syncthreads();
     for (int p = threadIdx.x; p < a.nparts; p += blockDim.x) {

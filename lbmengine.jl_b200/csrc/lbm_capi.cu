@@ -116,7 +116,10 @@ struct lbm_handle {
     int res_cluster = 0;                // CTAs per cluster; 0: one cooperative grid
     bool res_ready = false;             // the jobs below are current
     ResidentJob* d_rjobs = nullptr;     // [2]: by the buffer the first tick reads
-    unsigned *d_pmask = nullptr, *d_wmask = nullptr, *d_rbar = nullptr;
+    unsigned *d_pmask = nullptr, *d_wmask = nullptr;
+    int* d_rsync = nullptr;             // barrier counter and last phase, then the particles' boxes
+    double* d_rpos = nullptr;           // [2][particles][3]
+    int res_parts = 0;                  // particles the two hold
     void* pop[2] = {nullptr, nullptr};
     int cur = 0;
     double* d_coord[3] = {nullptr, nullptr, nullptr};
@@ -486,6 +489,7 @@ int ensure_tmp(lbm_handle* h, size_t bytes) {
 void drop_graphs(lbm_handle* h) {
     h->tick_ready = false;  // the tick kernel's maps and arguments are rebuilt with the graphs
     h->res_ready = false;
+    h->res_ctas = -1;
     for (auto& prof : h->graphs)
         for (auto& row : prof)
             for (auto& gr : row) {
@@ -810,39 +814,50 @@ int prepare_tick(lbm_handle* h) {
 // ---- many ticks per launch (resident.cuh) -----------------------------------
 
 // Grids that run resident, in nodes.  With a particle a resident tick takes
-// 3.1-4.3 us up to 2^17 nodes (the particle's chain) where the stream schedule
-// takes 9.3-11.4 us; from there on both grow with the grid, the stream schedule
-// more slowly (it moves four nodes per thread).  With walls alone 2.6 against
-// 5.0 us at 13,000 nodes, 6.1 against 6.9 at 255,000.  Plain fluid needs no
-// barrier beside the tick itself: 2.1 against 2.2 us on one cluster, and the
-// stream schedule is faster beyond (3.0 against 2.5 us at 100 x 100).
+// 3.4-4.6 us up to 2^17 nodes (the particle's chain) where the stream schedule
+// takes 9.2-11 us; from there on both grow with the grid, the stream schedule
+// more slowly (it moves four nodes per thread): 8.9 against 11.2 us at 724^2
+// FP32, 11.7 against 14.1 at 1024 x 512 FP64, 16.3 against 12.7 at 1024^2.  With
+// walls alone 2.6 against 5.0 us at 13,000 nodes, 6.1 against 6.9 at 255,000.
+// Plain fluid needs no barrier beside the tick itself: 2.1 against 2.2 us on
+// one cluster, and the stream schedule is level or faster beyond.
 constexpr long long kResidentNodesPart = 1ll << 19;
 constexpr long long kResidentNodesWalls = 1ll << 18;
 constexpr long long kResidentNodesFluid = (kResMaxCluster - 1) * kResThreads;
 constexpr int64_t kResidentTicks = 4096;  // ticks per launch
 
-// an upper bound of the link entries a particle of radius r (in nodes) can
-// have in 2D: the nodes less than sqrt(2) outside the sphere (their unit
-// squares lie in a ring), and those across the periodic boundary from a sphere
-// clipped at the edges of the box
-long long resident_entries(double r) {
-    const double s2 = std::sqrt(2.0), out = r + 1.5 * s2, in = std::max(0.0, r - 0.5 * s2);
-    return (long long)std::ceil(3.14159265358979 * (out * out - in * in) + 4.0 * (2.0 * r + 4.0));
-}
-long long resident_entries(const lbm_handle* h) {
-    long long e = 1;
-    for (const ParticleDev& P : h->hparts)
-        e = std::max(e, std::min<long long>(P.link_cap, resident_entries(P.radius / h->dx)));
-    return e;
+// Shared memory of a boundary CTA: bounds that no particle of its radius
+// exceeds (a cluster launch cannot end early).  The link nodes lie less than
+// sqrt(2) outside the sphere (their unit squares in a ring), or across the
+// periodic boundary from a sphere clipped at the edges of the box; eight slots
+// each.
+struct ResidentCaps {
+    long long entries = 1, slots = 1, box = 1;
+};
+ResidentCaps resident_caps(const lbm_handle* h) {
+    ResidentCaps c;
+    const double pi = 3.14159265358979;
+    for (const ParticleDev& P : h->hparts) {
+        const double r = P.radius / h->dx;
+        const double s2 = std::sqrt(2.0), out = r + 1.5 * s2, in = std::max(0.0, r - 0.5 * s2);
+        const double e = pi * (out * out - in * in) + 4.0 * (2.0 * r + 4.0);
+        c.entries = std::max(c.entries, std::min<long long>(P.link_cap, (long long)std::ceil(e)));
+        c.slots = std::max(c.slots, 8 * (long long)std::ceil(e));
+        for (int k = 0; k < h->dims; ++k)
+            c.box = std::max(c.box, std::min<long long>((long long)std::floor(2.0 * r) + 8, h->n[k]) + 2);
+    }
+    return c;
 }
 
-// dynamic shared memory per CTA
-size_t resident_smem(const lbm_handle* h) { return h->ops.resident_smem((int)resident_entries(h)); }
-
-// 2D, FP32 or FP64 storage, at most one particle, no interactions
+// 2D, FP32 or FP64 storage and few enough particles, links and interactions.
+// (In 3D the boundary CTA's FP64 work on some 500 entries and 3,000 slots is
+// the tick: 17.7 us against 11.8 in stream order for r = 5 in 32^3.)
 bool resident_applies(const lbm_handle* h) {
-    return h->ops.resident != nullptr && h->hparts.size() <= 1 && h->inter.empty() && h->d_rec == nullptr &&
-           resident_entries(h) <= kResMaxEntries && resident_smem(h) <= kResMaxSmem;
+    if (!h->ops.resident || h->d_rec || h->hparts.size() > (size_t)kResMaxParts) return false;
+    const ResidentCaps c = resident_caps(h);
+    return c.entries <= kResMaxEntries && c.box <= 1023 && c.slots < (1 << 20) &&
+           h->ops.resident_smem((int)c.entries, (int)c.slots, (int)c.box) <= kResMaxSmem &&
+           3 * h->inter.size() <= (size_t)kResMaxInter;
 }
 
 // how many clusters of `csize` CTAs with `smem` bytes of dynamic shared memory
@@ -877,25 +892,27 @@ bool use_resident(lbm_handle* h) {
         h->N > (!h->hparts.empty() ? kResidentNodesPart : (h->has_walls ? kResidentNodesWalls : kResidentNodesFluid)))
         return false;
     if (h->res_ctas < 0) {
-        // one node per thread, and a CTA for the particle: a cluster where that
-        // fits one, else a grid of one CTA per SM at most
-        const int want = (int)((h->N + kResThreads - 1) / kResThreads) + 1;
-        const size_t smem = kResMaxSmem;
+        // one node per thread, and a CTA per particle: a cluster where that
+        // fits one (one particle at most), else a grid of one CTA per SM at most
+        const int np = (int)h->hparts.size();
+        const int want = (int)((h->N + kResThreads - 1) / kResThreads) + np;
         h->res_ctas = 0;
         h->res_cluster = 0;
-        if (want <= kResMaxCluster && resident_clusters(h, smem, kResMaxCluster) > 0) {
+        if (np <= 1 && want <= kResMaxCluster &&
+            resident_clusters(h, kResMaxSmem, kResMaxCluster) > 0) {
             h->res_cluster = h->res_ctas = want <= 8 ? 8 : kResMaxCluster;
         } else {
             int sms = 0, per = 0, coop = 0;
-            resident_clusters(h, smem, 1);  // sets the kernel's shared-memory limit
+            resident_clusters(h, kResMaxSmem, 1);  // sets the kernel's shared-memory limit
             if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) == cudaSuccess &&
                 cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) == cudaSuccess && coop &&
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, h->ops.resident_fn, kResThreads, smem) == cudaSuccess)
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, h->ops.resident_fn, kResThreads, kResMaxSmem) ==
+                    cudaSuccess)
                 h->res_ctas = per > 0 ? std::min(want, sms) : 0;
             cudaGetLastError();
         }
     }
-    return h->res_ctas > 0;
+    return h->res_ctas > (int)h->hparts.size();
 }
 
 // the job of model h whose first tick reads buffer `src`
@@ -904,19 +921,29 @@ ResidentJob resident_job(const lbm_handle* h, int src) {
     for (int s = 0; s < 2; ++s) j.a[s] = step_args(h, src ^ s);
     j.pa = particle_args(h, 0, 0);  // publishes the box into both buffers
     j.pa.inline_links = 1;
+    j.in = inter_args(h);
     j.pmask = h->d_pmask;
     j.wmask = h->has_walls ? h->d_wmask : nullptr;
+    j.box = h->d_rsync + 2;
+    j.pos = h->d_rpos;
     return j;
 }
 
-// the masks of pushes a resident launch leaves out
-int resident_masks(lbm_handle* h) {
+// the device buffers of resident launches: masks of the pushes they leave out, jobs, barrier, particle boxes
+int resident_buffers(lbm_handle* h) {
     int rc = LBM_OK;
-    if (!h->d_pmask) {
-        rc = dev_alloc(h, &h->d_pmask, sizeof(unsigned) * h->N);
-        if (rc) return rc;
+    const int np = (int)h->hparts.size();
+    if (!h->d_pmask) rc = dev_alloc(h, &h->d_pmask, 2 * sizeof(unsigned) * h->N);
+    if (!rc && !h->d_rjobs) rc = dev_alloc(h, &h->d_rjobs, 2 * sizeof(ResidentJob));
+    if (!rc && (!h->d_rsync || h->res_parts < np)) {
+        dev_free(h->d_rsync);
+        dev_free(h->d_rpos);
+        rc = dev_alloc(h, &h->d_rsync, sizeof(int) * (2 + 6 * kResMaxParts));
+        if (!rc) rc = dev_alloc(h, &h->d_rpos, sizeof(double) * 6 * kResMaxParts);
+        h->res_parts = kResMaxParts;
     }
-    CUDA_TRY(h, cudaMemsetAsync(h->d_pmask, 0, sizeof(unsigned) * h->N, h->stream));
+    if (rc) return rc;
+    CUDA_TRY(h, cudaMemsetAsync(h->d_pmask, 0, 2 * sizeof(unsigned) * h->N, h->stream));
     if (h->has_walls && !h->d_wmask) {
         rc = dev_alloc(h, &h->d_wmask, sizeof(unsigned) * h->N);
         if (rc) return rc;
@@ -926,32 +953,42 @@ int resident_masks(lbm_handle* h) {
     return LBM_OK;
 }
 
-// nsteps ticks; the buffers swap roles after an odd number
-int resident_ticks(lbm_handle* h, int64_t nsteps) {
+// up to nsteps ticks; *ran: how many (fewer where a launch ended early).  The
+// buffers swap roles after an odd number.
+int resident_ticks(lbm_handle* h, int64_t nsteps, int64_t* ran) {
+    *ran = 0;
     if (!h->res_ready) {
-        int rc = resident_masks(h);
-        if (!rc && !h->d_rjobs) rc = dev_alloc(h, &h->d_rjobs, 2 * sizeof(ResidentJob));
-        if (!rc && !h->d_rbar) rc = dev_alloc(h, &h->d_rbar, sizeof(unsigned));
+        const int rc = resident_buffers(h);
         if (rc) return rc;
         const ResidentJob j[2] = {resident_job(h, 0), resident_job(h, 1)};
         CUDA_TRY(h, cudaMemcpyAsync(h->d_rjobs, j, sizeof(j), cudaMemcpyHostToDevice, h->stream));
         CUDA_TRY(h, cudaStreamSynchronize(h->stream));
         h->res_ready = true;
     }
-    for (int64_t done = 0; done < nsteps;) {
-        const int64_t n = std::min<int64_t>(kResidentTicks, nsteps - done);
+    const ResidentCaps caps = resident_caps(h);
+    const bool may_stop = h->hparts.size() > 1;  // a launch can end early
+    while (*ran < nsteps) {
+        int64_t n = std::min<int64_t>(kResidentTicks, nsteps - *ran);
         ResidentArgs r{};
         r.job = h->d_rjobs + h->cur;
         r.ticks = (int)n;
-        r.max_entries = (int)resident_entries(h);
+        r.cap_entries = (int)caps.entries;
+        r.cap_slots = (int)caps.slots;
+        r.cap_box = (int)caps.box;
         r.err = h->d_err;
         if (h->res_cluster == 0) {
-            r.bar = h->d_rbar;
-            CUDA_TRY(h, cudaMemsetAsync(h->d_rbar, 0, sizeof(unsigned), h->stream));
+            r.bar = reinterpret_cast<unsigned*>(h->d_rsync);
+            CUDA_TRY(h, cudaMemsetAsync(h->d_rsync, 0, sizeof(unsigned), h->stream));
+            CUDA_TRY(h, cudaMemsetAsync(h->d_rsync + 1, 0xff, sizeof(unsigned), h->stream));
         }
         CUDA_TRY(h, h->ops.resident(r, h->res_ctas, h->res_cluster, h->stream));
+        int phase = -1;  // the barrier phase the launch ended at (the first one lies before its first tick)
+        if (may_stop) CUDA_TRY(h, read_small(&phase, h->d_rsync + 1, sizeof(int), h->stream));
+        const bool stopped = phase >= 0;
+        if (stopped) n = phase - 1;
         if (n & 1) h->cur = 1 - h->cur;
-        done += n;
+        *ran += n;
+        if (stopped) break;
     }
     return LBM_OK;
 }
@@ -1224,7 +1261,8 @@ void destroy_all(lbm_handle* h) {
     dev_free(h->d_rjobs);
     dev_free(h->d_pmask);
     dev_free(h->d_wmask);
-    dev_free(h->d_rbar);
+    dev_free(h->d_rsync);
+    dev_free(h->d_rpos);
     dev_free(h->d_pargs);
     dev_free(h->d_tq);
     for (auto& e : h->pev) cudaEventDestroy(e);
@@ -1845,9 +1883,13 @@ int lbm_step(lbm_handle* h, int64_t nsteps) {
     int64_t done = 0;
     int slots_used = 0;
     if (resident) {
-        const int rc = resident_ticks(h, nsteps);
+        const int rc = resident_ticks(h, nsteps, &done);
         if (rc) return rc;
-        done = nsteps;
+        if (done < nsteps) {  // a launch ended early: the rest of the call in stream order
+            int rc2 = prepare_tick(h);
+            if (!rc2) rc2 = ensure_graphs(h, nsteps - done);
+            if (rc2) return rc2;
+        }
     }
     if (direct) {
         for (; done < nsteps; ++done) {

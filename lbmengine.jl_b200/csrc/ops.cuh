@@ -45,7 +45,7 @@ struct Ops {
     cudaError_t (*resident)(const ResidentArgs&, int ctas, int csize, cudaStream_t);
     void (*resident_wmask)(const unsigned char* wall, const GridDesc&, unsigned* wmask, cudaStream_t);
     const void* resident_fn;
-    size_t (*resident_smem)(int max_entries);  // dynamic shared memory per CTA
+    size_t (*resident_smem)(int entries, int slots, int box);  // dynamic shared memory per CTA
     // discrete adjoint of one tick, and of the initial condition (adjoint.cuh)
     void (*adjoint)(const AdjArgs&, unsigned link_ctas, cudaStream_t);  // link terms, then the nodes
     void (*adjoint_particle)(const AdjArgs&, cudaStream_t);
@@ -140,9 +140,8 @@ struct OpsImpl {
         }
     }
     static constexpr bool kResident = L::D == 2 && (ST == ST_F32 || ST == ST_F64);
-    static size_t resident_smem(int entries) {
-        if constexpr (kResident) return ResidentBoundary<L, ST>::bytes(entries);
-        return 0;
+    static size_t resident_smem(int entries, int slots, int box) {
+        return ResidentBoundary<ST>::bytes(entries, slots, box);
     }
     static void resident_wmask(const unsigned char* wall, const GridDesc& g, unsigned* wmask, cudaStream_t s) {
         k_resident_wmask<L><<<blocks_for(g.N, 256), 256, 0, s>>>(wall, g, wmask);
@@ -152,7 +151,7 @@ struct OpsImpl {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)ctas);
             cfg.blockDim = dim3(kResThreads);
-            cfg.dynamicSmemBytes = resident_smem(a.max_entries);
+            cfg.dynamicSmemBytes = resident_smem(a.cap_entries, a.cap_slots, a.cap_box);
             cfg.stream = s;
             cudaLaunchAttribute attr[1];
             if (csize > 0) {

@@ -23,8 +23,8 @@
 // equal bit for bit.
 //
 // Measured with a squirmer, per tick, against the stream schedule: 64^2 FP32
-// 3.1 us (9.4), 256 x 128 FP64 3.8 (10.2), 201 x 65 with walls 3.6 (10.4),
-// 512 x 256 FP32 3.9 (10.0).  The chain that bounds it: barrier and fence 1.0,
+// 3.4 us (9.2), 256 x 128 FP64 4.2 (9.9), 201 x 65 FP64 with walls 4.2 (11.1),
+// 512 x 256 FP32 4.4 (9.7), 724^2 FP32 8.9 (11.2).  The chain that bounds it: barrier and fence 1.0,
 // link nodes 0.8, slots and their sums 0.7, the verdict on the geometry 0.4 us.
 // (Two barriers per tick, with the slots stored between them over the pushes,
 // took 3.4 to 5.6 us for the same grids.)
@@ -36,29 +36,38 @@
 #pragma once
 #include "fixup.cuh"
 #include "particles.cuh"
+#include "interactions.cuh"
 
 namespace lbm {
 
 constexpr int kResThreads = 512;      // threads per CTA
 constexpr int kResHalf = 256;         // threads per chunk of link entries (= the fix-up's CTA: sums in the same order)
 constexpr int kResMaxCluster = 16;
-constexpr int kResMaxEntries = 1024;  // link entries of the particle, where their shared memory fits
-constexpr size_t kResMaxSmem = 200 * 1024;
-constexpr int kResMaxChunks = kResMaxEntries / kFixBlock;
+constexpr int kResMaxChunks = 32;                            // one lane per chunk in resident_sum
+constexpr int kResMaxEntries = kResMaxChunks * kFixBlock;    // link entries of a particle
+constexpr int kResMaxParts = 32;
+constexpr int kResMaxInter = 128;                            // interaction contributions to one particle
+constexpr size_t kResMaxSmem = 200 * 1024;                   // dynamic shared memory per CTA
 constexpr long long kResSpinLimit = 1LL << 22;  // polls of the grid barrier before it gives up (about a second)
 
 struct ResidentJob {
     StepArgs a[2];          // by tick parity
     ParticleArgs pa;
-    unsigned* pmask;        // [N] directions a node does not push: the particle's link slots (zero between launches)
+    InterArgs in;           // particle interactions (nitems 0: none)
+    unsigned* pmask;        // [2][N] directions a node does not push, the particles' link slots, by tick parity
+                            // (a geometry change of tick t goes to tick t + 1's mask while the bulk phase still
+                            // reads tick t's); zero between launches
     const unsigned* wmask;  // [N] the same for wall nodes and wall links (static), or null
+    int* box;               // [nparts][6] solid boxes, kept current while the launch runs
+    double* pos;            // [2][nparts][3] positions at the start of a tick, by its parity
 };
 
 struct ResidentArgs {
     const ResidentJob* job;
     int ticks;
-    int max_entries;     // link entries the boundary CTA's shared memory holds
-    unsigned* bar;       // grid barrier counter, zero at launch (null: cluster barrier)
+    int cap_entries, cap_slots, cap_box;  // shared memory of a boundary CTA (ResidentBoundary)
+    unsigned* bar;       // grid barrier: counter (zero at launch) and the phase the launch ends at (all
+                         // ones at launch); null: cluster barrier
     int* err;            // of the grid barrier
 };
 
@@ -92,17 +101,23 @@ __device__ __forceinline__ void cluster_wait() {
 
 // The barrier between ticks.  arrive(): after a __syncthreads that follows the
 // CTA's stores, by every thread; the last warp makes them visible and arrives
-// for the CTA.  wait(): by every thread; false when a bounded wait gave up
-// (every CTA then leaves at its next wait).
+// for the CTA.  stop (grid barrier only): every CTA leaves after this phase;
+// the counter's top bit says that some phase was named, the second word which
+// one (a CTA still waiting for an earlier phase must not leave at it).
+// wait(): by every thread; kGoOn, kStop, or kGaveUp when the bounded wait ran
+// out (every CTA then gives up at its next wait).
 struct ResidentBarrier {
+    enum { kGoOn = 0, kStop = 1, kGaveUp = 2 };
     unsigned* ctr;      // null: cluster barrier
     int* err;
-    unsigned target;    // arrivals that complete the current phase
+    unsigned phase;     // phases completed
     unsigned ctas;
-    __device__ __forceinline__ void arrive() {
+    __device__ __forceinline__ void arrive(bool stop = false) {
         if (ctr) {
             if (threadIdx.x == kResThreads - 32) {
+                if (stop) atomicMin(ctr + 1, phase + 1);
                 __threadfence();
+                if (stop) atomicOr(ctr, 0x80000000u);  // before the arrival: who sees the one sees the other
                 atomicAdd(ctr, 1u);
             }
         } else if (threadIdx.x >= kResThreads - 32) {
@@ -112,30 +127,37 @@ struct ResidentBarrier {
             cluster_arrive_relaxed();
         }
     }
-    __device__ __forceinline__ bool wait() {
+    static __device__ __forceinline__ unsigned load(const unsigned* p) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ int wait() {
+        ++phase;
         if (!ctr) {
             cluster_wait();
-            return true;
+            return kGoOn;
         }
-        target += ctas;
-        __shared__ int s_ok;
+        __shared__ int s_state;
         if (threadIdx.x == 0) {
-            int ok = 1;
+            int state = kGoOn;
             long long it = 0;
-            unsigned v;
             while (true) {
-                asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
-                if ((int)(v - target) >= 0) break;
+                const unsigned v = load(ctr);
+                if ((v & 0x7fffffffu) >= phase * ctas) {
+                    if ((v & 0x80000000u) && load(ctr + 1) <= phase) state = kStop;
+                    break;
+                }
                 if (++it > kResSpinLimit) {
                     atomicOr(err, kErrSpinTimeout);
-                    ok = 0;
+                    state = kGaveUp;
                     break;
                 }
             }
-            s_ok = ok;
+            s_state = state;
         }
         __syncthreads();
-        return s_ok != 0;
+        return s_state;
     }
 };
 
@@ -203,31 +225,47 @@ __device__ __forceinline__ bool resident_node(const StepArgs& a, const unsigned*
     return bad_density(rho);
 }
 
-// nodes first, first + stride, ... of the grid, two at a time: the loads of
-// both are in flight together
+// Nodes first, first + stride, ... of the grid; D2Q9 two at a time, so that the
+// loads of both are in flight together (the 3D sets fill the registers with one).
 template <class L, int ST, bool TRT, bool WALLS>
 __device__ __forceinline__ void resident_bulk(const StepArgs& a, const unsigned* pmask, const unsigned* wmask,
-                                              int first, int stride, int x, int y, int z, bool init) {
+                                              int first, int stride, int x, int y, int z, const int* step, bool init) {
     using R = typename Store<ST>::R;
     const int nx = a.g.n[0], ny = a.g.n[1], N = (int)a.g.N;
     bool bad = false;
-    for (int cell = first; cell < N; cell += 2 * stride) {
-        const int c2 = cell + stride;
-        const bool two = c2 < N;
-        R g[2][L::Q];
-        load_pops_l2<L, ST>(a, cell, g[0]);
-        load_pops_l2<L, ST>(a, two ? c2 : cell, g[1]);
-        if (cell != first) {
-            x = cell % nx;
-            y = L::D == 2 ? cell / nx : (cell / nx) % ny;
-            z = L::D == 2 ? 0 : cell / (nx * ny);
+    auto advance = [&]() {  // (x, y, z) of the node `stride` further on
+        x += step[0];
+        y += step[1];
+        z += step[2];
+        if (x >= nx) {
+            x -= nx;
+            ++y;
         }
-        bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, cell, x, y, z, g[0], init);
-        if (!two) break;
-        x = c2 % nx;
-        y = L::D == 2 ? c2 / nx : (c2 / nx) % ny;
-        z = L::D == 2 ? 0 : c2 / (nx * ny);
-        bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, c2, x, y, z, g[1], init);
+        if (L::D == 3 && y >= ny) {
+            y -= ny;
+            ++z;
+        }
+    };
+    if (L::Q <= 9) {
+        for (int cell = first; cell < N; cell += 2 * stride) {
+            const int c2 = cell + stride;
+            const bool two = c2 < N;
+            R g[2][L::Q];
+            load_pops_l2<L, ST>(a, cell, g[0]);
+            load_pops_l2<L, ST>(a, two ? c2 : cell, g[1]);
+            bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, cell, x, y, z, g[0], init);
+            if (!two) break;
+            advance();
+            bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, c2, x, y, z, g[1], init);
+            advance();
+        }
+    } else {
+        for (int cell = first; cell < N; cell += stride) {
+            R g[L::Q];
+            load_pops_l2<L, ST>(a, cell, g);
+            bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, cell, x, y, z, g, init);
+            advance();
+        }
     }
     if (bad) atomicOr(a.err, kErrNumeric);
 }
@@ -252,31 +290,37 @@ __global__ void k_resident_wmask(const unsigned char* wall, GridDesc g, unsigned
     wmask[c] = m;
 }
 
-// shared memory of the boundary CTA, in a fixed layout for `max_entries` entries
-template <class L, int ST>
+// Shared memory of a boundary CTA: capacities E (link entries), S (slots) and
+// B (nodes per axis of the near box and one more on each side).
+template <int ST>
 struct ResidentBoundary {
     using R = typename Store<ST>::R;
-    static constexpr int Q = L::Q, D = L::D;
-    int E;            // max_entries
-    double* C;        // [D][3][E] coordinates of x - 1, x, x + 1 per axis
-    double* rho;      // [E]
-    double* cu;       // [E Q] c_i . slip velocity of the slots' source nodes
-    R* g;             // [Q][E] post-collision populations (f/w - rho0)
+    int E, S, B;
+    double* cu;       // [S] c_i . slip velocity of the slots' source nodes
+    double* rho;      // [E] density of the entries
+    double* X;        // [3][B] node coordinates per axis, from slo - 2 on (periodic)
+    R* gi;            // [S] f*_i/w - rho0 of the slots' directions i = opp(j)
     int* cell;        // [E]
     int* mask;        // [E]
-    unsigned short* list;  // [E Q] (entry << 5) | j, chunk by chunk of kFixBlock entries
-    static __host__ __device__ size_t bytes(int E) {
-        return (size_t)E * (sizeof(double) * (3 * D + 1 + Q) + sizeof(R) * Q + 2 * sizeof(int) +
-                            sizeof(unsigned short) * Q);
+    int* loc;         // [E] position in the near box, 10 bits per axis
+    int* slot;        // [E] first slot
+    int* src;         // [2][S] source nodes whose pushes pmask leaves out, by tick parity
+    unsigned short* list;  // [S] (entry << 5) | j, chunk by chunk of kFixBlock entries
+    static __host__ __device__ size_t bytes(int E, int S, int B) {
+        return sizeof(double) * ((size_t)S + E + 3 * B) + sizeof(R) * (size_t)S +
+               sizeof(int) * (4 * (size_t)E + 2 * (size_t)S) + sizeof(unsigned short) * (size_t)S;
     }
-    __device__ __forceinline__ ResidentBoundary(unsigned char* p, int e) : E(e) {
-        C = reinterpret_cast<double*>(p);
-        rho = C + 3 * D * E;
-        cu = rho + E;
-        g = reinterpret_cast<R*>(cu + Q * E);
-        cell = reinterpret_cast<int*>(g + Q * E);
+    __device__ __forceinline__ ResidentBoundary(unsigned char* p, int e, int s, int b) : E(e), S(s), B(b) {
+        cu = reinterpret_cast<double*>(p);
+        rho = cu + S;
+        X = rho + E;
+        gi = reinterpret_cast<R*>(X + 3 * B);
+        cell = reinterpret_cast<int*>(gi + S);
         mask = cell + E;
-        list = reinterpret_cast<unsigned short*>(mask + E);
+        loc = mask + E;
+        slot = loc + E;
+        src = slot + E;
+        list = reinterpret_cast<unsigned short*>(src + 2 * S);
     }
 };
 
@@ -325,27 +369,29 @@ struct ResidentNew {
     double v[3], R[3], w[3], e[3], F[3], T[3];
     int moved, alpha, keep;
 };
-// the chunks' sums in the order of particles_core: a butterfly over 32 lanes of one chunk each
-__device__ __forceinline__ double resident_sum(const double (*part)[kPartialStride], int nch, int k) {
-    double v[kResMaxChunks];
+// the chunks' sums in the order of particles_core: a butterfly over the lanes of one chunk each (a whole warp)
+__device__ __forceinline__ double resident_sum(const double (*part)[kPartialStride], int nch, int k, int lane) {
+    static_assert(kResMaxChunks == 32, "one lane per chunk");
+    if (nch <= 2) return nch == 0 ? 0.0 : (nch == 1 ? part[0][k] : part[0][k] + part[1][k]);  // the same sum
+    double v = lane < nch ? part[lane][k] : 0.0;
 #pragma unroll
-    for (int c = 0; c < kResMaxChunks; ++c) v[c] = c < nch ? part[c][k] : 0.0;
-    // lanes 8, 4, 2, 1 apart; chunks past the list are zero
-#pragma unroll
-    for (int o = kResMaxChunks / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int c = 0; c < o; ++c) v[c] += v[c + o];
-    static_assert(kResMaxChunks <= 32, "one lane per chunk");
-    return v[0];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 template <int D>
 __device__ __forceinline__ void resident_translate(const ParticleArgs& a, const ParticleDev& P, const ResidentKeep& K,
                                                    const double (*part)[kPartialStride], int nch, int lane,
-                                                   ResidentNew* N) {
+                                                   const double* fint, ResidentNew* N) {
     const int k = lane & 3;  // lanes 4.. repeat lanes 0..3; component 3 (and 2 in 2D) is idle
     const bool on = k < D;
     const int q = on ? k : 0;
-    const double F = resident_sum(part, nch, q);
+    double F = 0.0;
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        const double f = resident_sum(part, nch, c, lane);
+        if (q == c) F = f;
+    }
+    if (fint) F += fint[q];  // the interactions' share of the force input
     const double dt = a.dt;
     double v = P.v[q], R = P.R[q];
     bool moved = false;
@@ -381,7 +427,7 @@ __device__ __forceinline__ void resident_rotate(const ParticleArgs& a, const Par
     constexpr int NW = D == 2 ? 1 : 3;
     double T[3] = {0, 0, 0}, w[3] = {P.w[0], P.w[1], P.w[2]}, e[3] = {P.e[0], P.e[1], P.e[2]};
 #pragma unroll
-    for (int k = 0; k < NW; ++k) T[k] = resident_sum(part, nch, 3 + k);
+    for (int k = 0; k < NW; ++k) T[k] = resident_sum(part, nch, 3 + k, lane);
     const double dt = a.dt;
     bool alpha = false;
     if (P.rules == 1) {
@@ -413,7 +459,8 @@ __device__ __forceinline__ void resident_rotate(const ParticleArgs& a, const Par
 }
 // the kept update into the record, by one warp
 template <int D>
-__device__ __forceinline__ void resident_commit(const ParticleArgs& a, ParticleDev& P, const ResidentNew& N, int lane) {
+__device__ __forceinline__ void resident_commit(const ParticleArgs& a, int p, ParticleDev& P, const ResidentNew& N,
+                                                int lane) {
     constexpr int NW = D == 2 ? 1 : 3;
     const bool nv = N.moved || N.alpha;  // getNodeVelocity: the snapshot of the slip velocity
     if (lane < D) {
@@ -441,7 +488,7 @@ __device__ __forceinline__ void resident_commit(const ParticleArgs& a, ParticleD
     }
     __syncwarp();
     if (lane == 0 && a.trj) {
-        double* r = a.trj + (P.nrec % a.trj_cap) * a.nparts * 9;
+        double* r = a.trj + ((P.nrec % a.trj_cap) * a.nparts + p) * 9;
         for (int q = 0; q < 3; ++q) {
             r[q] = P.R[q];
             r[3 + q] = P.v[q];
@@ -473,8 +520,27 @@ __device__ __forceinline__ void resident_exchange(const StepArgs& a, const Parti
     }
 }
 
+// do the periodic index ranges of the near box of `b` grown by two nodes and the
+// near box of `o` meet (boxes as lo[3], hi[3] of the solid nodes)?
+template <int D>
+__device__ __forceinline__ bool resident_close(const int* b, const int* o, const int* n) {
+    bool meet = true;
+    for (int k = 0; k < D; ++k) {
+        if (b[k] > b[3 + k] || o[k] > o[3 + k]) return true;  // an empty region: left to the general path
+        meet = meet && ranges_meet(b[k] - 3, b[3 + k] - b[k] + 7, o[k] - 1, o[3 + k] - o[k] + 3, n[k]);
+    }
+    return meet;
+}
+
 // One CTA per SM (128 registers): the chain of latencies gains nothing from
-// occupancy.
+// occupancy.  The last nparts CTAs are the particles' boundary CTAs.
+//
+// With several particles each must be alone (no other particle's near box close
+// to its own) with links in every direction, so that a slot belongs to one
+// particle; a boundary CTA that finds otherwise, or whose links outgrow its
+// shared memory, ends the launch after the tick (the caller goes on with the
+// stream schedule).  Boxes of the others are read while they may be moving: by
+// at most a node per tick, which the margin of two nodes covers.
 template <class L, int ST, bool TRT>
 __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_constant__ ResidentArgs ra) {
     using SS = Store<ST>;
@@ -482,20 +548,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
     using R = typename SS::R;
     constexpr int Q = L::Q, D = L::D;
     constexpr int kHalves = kResThreads / kResHalf;
+    constexpr unsigned kAllDirs = (Q == 32 ? 0u : (1u << Q)) - 2u;
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ StepArgs s_a[2];
     __shared__ ParticleArgs s_pa;
-    __shared__ unsigned *s_pmask;
-    __shared__ const unsigned* s_wmask;
     __shared__ ParticleDev sP;
     __shared__ ResidentKeep s_keep;
     __shared__ ResidentNew s_new;
     __shared__ double s_part[kResMaxChunks][kPartialStride];
     __shared__ double s_red[kResThreads / 32][6];
     __shared__ int s_off[kResMaxChunks + 1];  // first slot of each chunk
-    __shared__ int s_wcnt[2];
+    __shared__ int s_wcnt[2], s_stop, s_box[6];
+    __shared__ int s_nsrc[2];  // source nodes set in each parity's pmask
     __shared__ int s_lat[4][Q];  // c_i (3) and i of the slot direction j, i = opp(j)
     __shared__ double s_w[Q];
+    __shared__ double s_fi[kResMaxInter][3], s_fint[3];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool grid = ra.bar != nullptr;
     const int rank = grid ? (int)blockIdx.x : (int)cluster_rank();
@@ -513,21 +580,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
         reinterpret_cast<int*>(s_a)[k] = reinterpret_cast<const int*>(J.a)[k];
     for (int k = tid; k < (int)(sizeof(ParticleArgs) / 4); k += kResThreads)
         reinterpret_cast<int*>(&s_pa)[k] = reinterpret_cast<const int*>(&J.pa)[k];
-    if (tid == 0) {
-        s_pmask = J.pmask;
-        s_wmask = J.wmask;
-    }
+    if (tid == 0) s_stop = s_nsrc[0] = s_nsrc[1] = 0;
     __syncthreads();
-    const bool part = s_a[0].nparts > 0;
+    const int np = s_a[0].nparts;
     const bool walls = s_a[0].nwnodes > 0;
-    const int bulk_ctas = part && csize > 1 ? csize - 1 : csize;
-    const bool does_bulk = rank < bulk_ctas, boundary = part && rank == csize - 1;
+    const int bulk_ctas = csize - np;
+    const bool boundary = rank >= bulk_ctas;
+    const int p = rank - bulk_ctas;  // the boundary CTA's particle
     const int nx = s_a[0].g.n[0], ny = s_a[0].g.n[1], nz = s_a[0].g.n[2];
-    unsigned* pmask = part ? s_pmask : nullptr;
-    const unsigned* wmask = s_wmask;
+    const long long N = s_a[0].g.N;
+    unsigned* const pmask = np > 0 ? J.pmask : nullptr;
+    const unsigned* const wmask = J.wmask;
     const int first = rank * kResThreads + tid, stride = bulk_ctas * kResThreads;
     const int x0 = first % nx, y0 = D == 2 ? first / nx : (first / nx) % ny, z0 = D == 2 ? 0 : first / (nx * ny);
-    ResidentBoundary<L, ST> B(s_dyn, ra.max_entries);
+    const int step[3] = {stride % nx, D == 2 ? stride / nx : (stride / nx) % ny, D == 2 ? 0 : stride / (nx * ny)};
+    ResidentBoundary<ST> B(s_dyn, ra.cap_entries, ra.cap_slots, ra.cap_box);
     int entries = 0, nch = 0;
     // the source node of slot `item` (the node pushed from by plain streaming)
     auto source = [&](int item) -> int {
@@ -536,31 +603,74 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
         const int z = D == 2 ? 0 : wrap_idx(cell / (nx * ny) + s_lat[2][j], nz);
         return x + nx * (y + ny * z);
     };
-    // entries, coordinates and slot list of the current links, and pmask with them
-    auto relist = [&]() {
-        const int old = nch > 0 ? s_off[nch] : 0;
-        for (int l = tid; l < old; l += kResThreads) pmask[source(B.list[l])] = 0u;
+    auto slots = [&]() -> int { return nch > 0 ? s_off[nch] : 0; };
+    // pmask of parity b: cleared, and set for the current slots
+    auto unmask = [&](int b) {
+        for (int l = tid; l < s_nsrc[b]; l += kResThreads) pmask[(size_t)b * N + B.src[b * B.S + l]] = 0u;
+    };
+    auto set_mask = [&](int b) {
+        unmask(b);
         __syncthreads();
+        const int now = slots();
+        for (int l = tid; l < now; l += kResThreads) {
+            const int item = B.list[l], at = source(item);
+            B.src[b * B.S + l] = at;
+            atomicOr(pmask + (size_t)b * N + at, 1u << (item & 31));
+        }
+        if (tid == 0) s_nsrc[b] = now;
+    };
+    // Entries, coordinates and slot list of the current links; sets s_stop
+    // where this launch cannot go on with them.
+    auto relist = [&](bool check_move) {
         const int nl = sP.nlinks;
-        entries = min(nl, B.E);
-        if (nl > B.E && tid == 0) atomicOr(s_a[0].err, kErrLinkOverflow);
+        bool fits = nl <= B.E;
+        const int ex = near_extent(sP, s_a[0].g, 0, D), ey = near_extent(sP, s_a[0].g, 1, D),
+                  ez = near_extent(sP, s_a[0].g, 2, D);
+        fits = fits && ex + 2 <= B.B && ey + 2 <= B.B && ez + 2 <= B.B;
+        entries = fits ? nl : 0;
         nch = (entries + kFixBlock - 1) / kFixBlock;
         for (int e = tid; e < entries; e += kResThreads) {
             const int2 ent = s_a[0].links[sP.link_off + e];
             B.cell[e] = ent.x;
             B.mask[e] = ent.y;
             const int xyz[3] = {ent.x % nx, (ent.x / nx) % ny, ent.x / (nx * ny)};
+            int loc = 0;
 #pragma unroll
-            for (int k = 0; k < D; ++k)
+            for (int k = 0; k < D; ++k) {
+                const int n = s_a[0].g.n[k], l = xyz[k] - (sP.slo[k] - 1);
+                loc |= (l < 0 ? l + n : (l >= n ? l - n : l)) << (10 * k);
+            }
+            B.loc[e] = loc;
+        }
+        if (entries > 0) {
 #pragma unroll
-                for (int o = 0; o < 3; ++o)
-                    B.C[(k * 3 + o) * B.E + e] = s_a[0].coord[k][wrap_idx(xyz[k] + o - 1, s_a[0].g.n[k])];
+            for (int k = 0; k < D; ++k) {
+                const int n = s_a[0].g.n[k];
+                for (int i = tid; i < near_extent(sP, s_a[0].g, k, D) + 2; i += kResThreads)
+                    B.X[k * B.B + i] = s_a[0].coord[k][((sP.slo[k] - 2 + i) % n + n) % n];
+            }
         }
         if (tid == 0) {
             s_off[0] = 0;
             resident_keep<D>(s_pa, sP, &s_keep);
+            if (!fits) s_stop = 1;
+            if (np > 1) {
+                if ((sP.dirlinks & kAllDirs) != kAllDirs) s_stop = 1;
+                for (int k = 0; k < 3; ++k) {
+                    // more than a node per tick: the margin does not hold
+                    if (check_move && (abs(sP.slo[k] - s_box[k]) > 1 || abs(sP.shi[k] - s_box[3 + k]) > 1)) s_stop = 1;
+                    s_box[k] = sP.slo[k];
+                    s_box[3 + k] = sP.shi[k];
+                }
+                for (int k = 0; k < 6; ++k) __stcg(J.box + 6 * p + k, s_box[k]);
+            }
         }
         __syncthreads();
+        if (np > 1 && tid < np && tid != p) {
+            int o[6];
+            for (int k = 0; k < 6; ++k) o[k] = __ldcg(J.box + 6 * tid + k);
+            if (resident_close<D>(s_box, o, s_a[0].g.n)) s_stop = 1;
+        }
         for (int c = 0; c < nch; ++c) {  // slots in entry order, as fixup_body lists them
             const int e = c * kFixBlock + tid;
             const unsigned mask = tid < kFixBlock && e < entries ? (unsigned)B.mask[e] : 0u;
@@ -575,24 +685,32 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                 if (lane == 31) s_wcnt[tid >> 5] = off;
             }
             __syncthreads();
+            const int base = s_off[c], end = base + s_wcnt[0] + s_wcnt[1];
+            if (end > B.S) {  // the same in every thread
+                if (tid == 0) s_stop = 1;
+                entries = 0;
+                nch = 0;
+                break;
+            }
             if (tid < kFixBlock) {
-                off += s_off[c] - cnt + (tid >= 32 ? s_wcnt[0] : 0);
+                off += base - cnt + (tid >= 32 ? s_wcnt[0] : 0);
+                if (e < entries) B.slot[e] = off;
                 for (unsigned m = mask; m; m &= m - 1) B.list[off++] = (unsigned short)((e << 5) | (__ffs(m) - 1));
             }
-            if (tid == 0) s_off[c + 1] = s_off[c] + s_wcnt[0] + s_wcnt[1];
+            if (tid == 0) s_off[c + 1] = end;
             __syncthreads();
         }
-        const int now = nch > 0 ? s_off[nch] : 0;
-        for (int l = tid; l < now; l += kResThreads) atomicOr(pmask + source(B.list[l]), 1u << (B.list[l] & 31));
+        __syncthreads();
     };
+    // the coordinate of entry e's node along axis k, o nodes further on
+    auto coord = [&](int e, int k, int o) -> double { return B.X[k * B.B + (B.loc[e] >> (10 * k) & 1023) + 1 + o]; };
     // c_i . slip velocity at every slot's source node, for the record's snapshot
     auto slip = [&]() {
-        const int now = nch > 0 ? s_off[nch] : 0;
+        const int now = slots();
         for (int l = tid; l < now; l += kResThreads) {
             const int item = B.list[l], e = item >> 5, j = item & 31;
             const int ci0 = s_lat[0][j], ci1 = s_lat[1][j], ci2 = s_lat[2][j];
-            const double Tc[3] = {B.C[(1 + ci0) * B.E + e], B.C[(4 + ci1) * B.E + e],
-                                  D == 3 ? B.C[(7 + ci2) * B.E + e] : 0.0};
+            const double Tc[3] = {coord(e, 0, ci0), coord(e, 1, ci1), D == 3 ? coord(e, 2, ci2) : 0.0};
             double up[3];
             if (sP.rules == 1)
                 slip_velocity_cpu<D>(sP.sR, sP.sV, sP.sW, sP.sE, sP.B1, sP.B2, sP.kind, sP.radius,
@@ -602,35 +720,80 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             B.cu[l] = ci0 * up[0] + ci1 * up[1] + ci2 * up[2];
         }
     };
+    const int ninter = boundary && J.in.nitems > 0 ? J.in.coff[p + 1] - J.in.coff[p] : 0;
     if (boundary) {
-        const unsigned long long* from = reinterpret_cast<const unsigned long long*>(s_pa.parts);
+        const unsigned long long* from = reinterpret_cast<const unsigned long long*>(s_pa.parts + p);
         for (int k = tid; k < (int)(sizeof(ParticleDev) / 8); k += kResThreads)
             reinterpret_cast<unsigned long long*>(&sP)[k] = from[k];
         __syncthreads();
-        if (tid == 0) s_pa.partial = &s_part[0][0] - (long long)sP.part_off * kPartialStride;  // from part_off on
-        relist();
+        if (tid == 0) {  // the CTA's own partial sums and interaction force, indexed as the global arrays
+            s_pa.partial = &s_part[0][0] - (long long)sP.part_off * kPartialStride;
+            s_pa.fint = J.in.nitems > 0 ? s_fint - 3 * p : nullptr;
+        }
+        if (tid < 3) __stcg(J.pos + 3 * p + tid, sP.R[tid]);
+        if (tid < np && tid != p) {  // the others as the launch finds them
+            const ParticleDev& O = s_pa.parts[tid];
+            const int b[6] = {sP.slo[0], sP.slo[1], sP.slo[2], sP.shi[0], sP.shi[1], sP.shi[2]};
+            const int o[6] = {O.slo[0], O.slo[1], O.slo[2], O.shi[0], O.shi[1], O.shi[2]};
+            if ((O.dirlinks & kAllDirs) != kAllDirs || resident_close<D>(b, o, s_a[0].g.n)) s_stop = 1;
+            for (int k = 0; k < 6; ++k) __stcg(J.box + 6 * tid + k, o[k]);  // every CTA writes the same
+        }
+        __syncthreads();
+        relist(false);
+        set_mask(0);
+        set_mask(1);
         slip();
         __syncthreads();
     }
-    if (part) {  // pmask is set before the first push
-        bar.arrive();
-        if (!bar.wait()) return;
+    bool stale = false;  // the other parity's mask is that of the links before the last change
+    int t = 0, state = ResidentBarrier::kGoOn;
+    if (np > 0) {  // pmask is set before the first push
+        bar.arrive(s_stop != 0);
+        state = bar.wait();
     }
-    for (int t = 0; t < ra.ticks; ++t) {
+    for (; t < ra.ticks && state == ResidentBarrier::kGoOn; ++t) {
         const StepArgs& a = s_a[t & 1];
-        if (does_bulk) {
-            if (walls) resident_bulk<L, ST, TRT, true>(a, pmask, wmask, first, stride, x0, y0, z0, t < 2);
-            else resident_bulk<L, ST, TRT, false>(a, pmask, wmask, first, stride, x0, y0, z0, false);
-        }
-        if (boundary) {
+        if (!boundary) {
+            const unsigned* pm = pmask ? pmask + (size_t)(t & 1) * N : nullptr;
+            if (walls) resident_bulk<L, ST, TRT, true>(a, pm, wmask, first, stride, x0, y0, z0, step, t < 2);
+            else resident_bulk<L, ST, TRT, false>(a, pm, wmask, first, stride, x0, y0, z0, step, false);
+            __syncthreads();
+            bar.arrive();
+        } else {
             // the link nodes, collided from src
             for (int e = tid; e < entries; e += kResThreads) {
                 R g[Q];
                 const int cell = B.cell[e];
+                const unsigned mask = (unsigned)B.mask[e];
                 load_pops_l2<L, ST>(a, cell, g);
                 B.rho[e] = (double)collide_node<L, ST, TRT>(a, cell, true, g);
+                int l = B.slot[e];
 #pragma unroll
-                for (int i = 0; i < Q; ++i) B.g[i * B.E + e] = g[i] * R(a.inv_scale);
+                for (int j = 1; j < Q; ++j)
+                    if (mask >> j & 1u) B.gi[l++] = g[L::opp(j)] * R(a.inv_scale);
+            }
+            if (J.in.nitems > 0) {  // interactions: the positions at the start of the tick (interactions.cuh)
+                const double* pos = J.pos + (size_t)(t & 1) * 3 * np;
+                if (tid >= kResThreads - kResMaxInter && tid - (kResThreads - kResMaxInter) < ninter) {
+                    const int q = tid - (kResThreads - kResMaxInter);
+                    const int c = J.in.cent[J.in.coff[p] + q];
+                    const InterItem it = J.in.items[c >> 3];
+                    double R1[3], R2[3], R3[3], out[9];
+                    for (int k = 0; k < 3; ++k) {
+                        R1[k] = __ldcg(pos + 3 * it.id1 + k);
+                        R2[k] = __ldcg(pos + 3 * it.id2 + k);
+                        R3[k] = it.kind == 2 ? __ldcg(pos + 3 * it.id3 + k) : 0.0;
+                    }
+                    interaction_force(it, D, R1, R2, R3, out);
+                    const double* v = out + 3 * (c >> 1 & 3);
+                    for (int k = 0; k < 3; ++k) s_fi[q][k] = c & 1 ? -v[k] : v[k];
+                }
+                __syncthreads();
+                if (tid < 3) {
+                    double f = 0.0;
+                    for (int q = 0; q < ninter; ++q) f += s_fi[q][tid];
+                    s_fint[tid] = f;
+                }
             }
             __syncthreads();
             // slot values, stored at once (nobody else writes them), and the momentum exchange:
@@ -645,7 +808,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                         const int item = B.list[l], e = item >> 5, j = item & 31, cell = B.cell[e];
                         if (walls && a.wall[cell]) continue;  // wall nodes hold f = 0 (fluids.jl:154)
                         const int ci[3] = {s_lat[0][j], s_lat[1][j], s_lat[2][j]};
-                        const double rhoL = B.rho[e], gi = (double)B.g[s_lat[3][j] * B.E + e];
+                        const double rhoL = B.rho[e], gi = (double)B.gi[l];
                         double v = gi;  // halfway bounce-back: f_j(x) = f*_i(x)
                         if (a.uw) {     // moving walls (fluids.jl:168-174)
                             const int q = source(item);
@@ -656,7 +819,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                         if (sP.dirlinks >> j & 1u) {
                             v += 6.0 * rhoL * -B.cu[l];
                             if (sP.coupleF || sP.coupleT || sP.recordF) {
-                                const double Xc[3] = {B.C[B.E + e], B.C[4 * B.E + e], D == 3 ? B.C[7 * B.E + e] : 0.0};
+                                const double Xc[3] = {coord(e, 0, 0), coord(e, 1, 0), D == 3 ? coord(e, 2, 0) : 0.0};
                                 resident_exchange<D>(a, sP, ci, Xc, gi, s_w[j], v, acc);
                             }
                         }
@@ -680,34 +843,47 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                 }
                 __syncthreads();
             }
-            if (warp == 0) resident_translate<D>(s_pa, sP, s_keep, s_part, nch, lane, &s_new);
-            else if (warp == 1) resident_rotate<D>(s_pa, sP, s_part, nch, lane, &s_new);
+            if (warp == 0)
+                resident_translate<D>(s_pa, sP, s_keep, s_part, nch, lane, J.in.nitems > 0 ? s_fint : nullptr, &s_new);
+            else if (warp == 1)
+                resident_rotate<D>(s_pa, sP, s_part, nch, lane, &s_new);
             __syncthreads();
+            double* next = J.pos + (size_t)((t + 1) & 1) * 3 * np + 3 * p;
             if (!s_new.keep) {  // the geometry may change: the full update, and pmask before the barrier
-                if (particles_core<L, 128>(s_pa, 0, sP)) {
-                    __syncthreads();
-                    relist();
-                }
+                const bool changed = particles_core<L, 128>(s_pa, p, sP);
                 __syncthreads();
-                bar.arrive();
+                if (changed) relist(true);
+                if (changed || stale) set_mask((t + 1) & 1);
+                stale = changed;
+                if (tid < 3) __stcg(next + tid, sP.R[tid]);
+                __syncthreads();
+                bar.arrive(s_stop != 0);
             } else {
+                if (stale) {
+                    set_mask((t + 1) & 1);
+                    stale = false;
+                    __syncthreads();
+                }
+                if (J.in.nitems > 0) {
+                    if (tid < D) __stcg(next + tid, s_new.R[tid]);
+                    else if (tid < 3) __stcg(next + tid, 0.0);
+                    __syncthreads();
+                }
                 bar.arrive();
-                if (warp == 0) resident_commit<D>(s_pa, sP, s_new, lane);
+                if (warp == 0) resident_commit<D>(s_pa, p, sP, s_new, lane);
             }
             __syncthreads();
             slip();
-        } else {
-            __syncthreads();
-            bar.arrive();
         }
-        if (!bar.wait()) return;
+        state = bar.wait();
     }
+    if (state == ResidentBarrier::kGaveUp) return;
     if (boundary) {  // pmask back to zero, the record back to global memory
         __syncthreads();
-        const int now = nch > 0 ? s_off[nch] : 0;
-        for (int l = tid; l < now; l += kResThreads) pmask[source(B.list[l])] = 0u;
-        store_record(s_pa, 0, sP);
-        if (tid == 0) publish_box(s_pa, 0, sP);
+        unmask(0);
+        unmask(1);
+        store_record(s_pa, p, sP);
+        if (tid == 0) publish_box(s_pa, p, sP);
     }
 }
 

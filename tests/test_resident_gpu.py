@@ -25,12 +25,18 @@ CASES = {
     # clipped at the domain's edge: the full update in every tick, links across the periodic boundary
     "clipped": dict(n=(64, 48), sq=dict(position=[-28.2, 0.1])),
     # more link entries than one chunk, than two, and than eight
-    "chunks": dict(n=(128, 96), sq=dict(radius=14.5)), "many_chunks": dict(n=(300, 260), sq=dict(radius=80.0), ticks=(1, 6)),
+    "chunks": dict(n=(128, 96), sq=dict(radius=14.5)), "many_chunks": dict(n=(300, 260), sq=dict(radius=45.0), ticks=(1, 6)),
     "held": dict(n=(64, 64), sq=dict(coupleForces=False, coupleTorques=False)),
     "walls": dict(n=(40, 33), walls=True), "walls_bead": dict(n=(201, 65), walls=True, kind="bead"),
     # a particle that overlaps the moving wall: slots that are wall links too
     "overlaps_lid": dict(n=(64, 33), walls=True, lid=True, sq=dict(position=[0.3, 11.2]), ticks=(1, 3, 12)),
     "walls_only": dict(n=(61, 40), walls=True, lid=True, kind=None), "fluid": dict(n=(64, 64), kind=None),
+    # a bulk phase longer than the boundary work, with the geometry changing under it
+    "long_bulk": dict(n=(700, 640), sq=dict(position=[0.499, 0.4996], swimmingSpeed=5e-3), ticks=(1, 40, 41)),
+    # several particles: bonded and repelling; two that come close end the launch; two apart
+    "bonded": dict(n=(120, 90), parts=[[-20.3, 0.2], [14.1, 0.6], [0.2, 27.4]], bonds=True),
+    "come_close": dict(n=(96, 64), parts=[[-9.6, 0.0], [9.4, 0.3]], toward=True, ticks=(1, 60, 61)),
+    "touching": dict(n=(96, 64), parts=[[-7.2, 0.0], [7.4, 0.3]], ticks=(1, 20)),
     "force": dict(n=(64, 40), force=[1e-5, 2e-6]), "force_field": dict(n=(65, 40), force="field"),
 }
 
@@ -54,6 +60,15 @@ def _model(case, schedule):
     m = lbm.modelInit(**kw)
     kind = case.get("kind", "squirmer")
     p = dict(SQ, **case.get("sq", {}))
+    if "parts" in case:
+        for k, pos in enumerate(case["parts"]):
+            e = [1.0 - 2.0 * k, 0.0] if case.get("toward") else [0.8, 0.6]
+            lbm.addSquirmer(m, **dict(p, position=pos, swimmingDirection=e, swimmingSpeed=8e-3 if case.get("toward") else 1e-3))
+        if case.get("bonds"):
+            lbm.addLinearBond(m, 1, 2, equilibriumDisplacement=36.0, stiffness=1e-2)
+            lbm.addPolarBond(m, 1, 3, 2, stiffness=1e-2)
+            lbm.addWCA(m)
+        return m
     if kind == "bead":
         p = {k: v for k, v in p.items() if k not in ("swimmingSpeed", "beta", "swimmingDirection")}
         lbm.addBead(m, velocity=[1e-3, -5e-4], **p)
@@ -78,9 +93,9 @@ def test_resident_matches_stream(lib, name):
                 u, v = np.array(getattr(p, f)), np.array(getattr(q, f))
                 scale = max(1.0 if f in ("position", "swimming_direction") else 1e-3, float(np.abs(v).max()))
                 assert np.abs(u - v).max() <= 1e-12 * scale + (1e-9 if tol > 1e-10 else 0) * scale, (f, u, v)
-        if case.get("kind", "squirmer"):
-            np.testing.assert_array_equal(a.solid_region(1), b.solid_region(1))
-            for u, v in zip(a.boundary_links(1), b.boundary_links(1)):
+        for pid in range(1, len(a.particle_states()) + 1):
+            np.testing.assert_array_equal(a.solid_region(pid), b.solid_region(pid))
+            for u, v in zip(a.boundary_links(pid), b.boundary_links(pid)):
                 np.testing.assert_array_equal(u, v)
     a.close()
     b.close()
