@@ -108,6 +108,15 @@ struct CollideK {
     R gA[27], gB[27];
 };
 
+// The FP32 constants of the collision twice in a row, as the two halves of the
+// packed instructions want them (collide_x2)
+struct CollideK2 {
+    float2 S, invS, rho0, rho_inc;
+    float2 hF[3], F[3];  // half_dt F, F
+    float2 rest, hsum, le, lo, omE, c45, c3, gK0;
+    float2 gA[27], gB[27];
+};
+
 struct StepArgs {
     const void* src;
     void* dst;
@@ -155,6 +164,7 @@ struct StepArgs {
     int reverse;                          // the vector bulk pass walks its tiles last to first (see k_bulk_v4)
     CollideK<float> kf;                   // the constants in FP32 and FP64 (fill_collide_consts)
     CollideK<double> kd;
+    CollideK2 k2;                         // kf, doubled
     // per-direction population planes of src / dst (vector bulk kernel)
     const void* srcq[27];
     void* dstq[27];
@@ -190,6 +200,29 @@ inline void fill_collide_k(const StepArgs& a, CollideK<R>& k) {
 inline void fill_collide_consts(StepArgs& a) {
     fill_collide_k(a, a.kf);
     fill_collide_k(a, a.kd);
+    auto two = [](float v) { return make_float2(v, v); };
+    const CollideK<float>& f = a.kf;
+    CollideK2& k = a.k2;
+    k.S = two(f.S);
+    k.invS = two(f.invS);
+    k.rho0 = two(f.rho0);
+    k.rho_inc = two(f.rho_inc);
+    for (int i = 0; i < 3; ++i) {
+        k.hF[i] = two(f.hdt * f.F[i]);
+        k.F[i] = two(f.F[i]);
+    }
+    k.rest = two(f.rest);
+    k.hsum = two(f.hsum);
+    k.le = two(f.le);
+    k.lo = two(f.lo);
+    k.omE = two(f.omE);
+    k.c45 = two(f.c45);
+    k.c3 = two(f.c3);
+    k.gK0 = two(f.gK0);
+    for (int i = 0; i < 27; ++i) {
+        k.gA[i] = two(f.gA[i]);
+        k.gB[i] = two(f.gB[i]);
+    }
 }
 
 template <class R>
@@ -442,6 +475,138 @@ __device__ __forceinline__ R collide(const StepArgs& a, R* g, R Fx, R Fy, R Fz, 
     return collide_sd<L, R, TRT>(a, g, s, d, Fx, Fy, Fz, field);
 }
 
+// ---------------------------------------------------------------------------
+// The collision of two nodes at once with the packed FP32 instructions of
+// sm_100 (one issue slot for two IEEE operations, each rounded as the scalar
+// one): collide() for two neighbouring nodes, operation by operation, so that
+// both give the same bits.  The 2-byte vector bulk pass was bound by issue
+// slots (71 % active, 285 instructions per D3Q19 node, half of them this
+// arithmetic), the FP32 one partly.  128^3 D3Q19: FP16 29.6 -> 28.6 us (18.6 ->
+// 13.0 M warp instructions; now the latency of its loads at 16 warps per SM),
+// FP32 46.2 -> 45.0; D3Q15 FP16 26.4 -> 24.3; D3Q27 FP32 69.2 -> 66.8; 192^3
+// D3Q19 BF16 96.5 -> 93.9.
+// ---------------------------------------------------------------------------
+using f32x2 = unsigned long long;  // lower half: the first node
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ f32x2 pack2(const float2& v) { return pack2(v.x, v.y); }
+__device__ __forceinline__ float low2(f32x2 v) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    return lo;
+}
+__device__ __forceinline__ float high2(f32x2 v) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    return hi;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// the member of a pair (i, opp(i)) whose first non-zero component is +1: taken
+// as the pair's first, c.u needs no negation (swapping the two flips the signs
+// of d, A, B and O exactly)
+template <class L>
+__host__ __device__ constexpr bool pair_leads(int i) {
+    return L::cx(i) != 0 ? L::cx(i) > 0 : (L::cy(i) != 0 ? L::cy(i) > 0 : L::cz(i) > 0);
+}
+
+// In: s[i] = g_i + g_opp, d[i] = g_i - g_opp for the leading i of each pair,
+// g[0] (and for BGK every g).  Out: g.  rho: the two densities.
+template <class L, bool TRT>
+__device__ __forceinline__ void collide_x2(const StepArgs& a, f32x2* g, const f32x2* s, const f32x2* d, float* rho) {
+    constexpr int Q = L::Q;
+    const CollideK2& k = a.k2;
+    f32x2 drho = pack2(0.f, 0.f), j[3] = {drho, drho, drho};
+    // in the order of collide(): the pairs by their smaller index
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int qb = L::opp(q);
+        if (qb < q) continue;
+        const float w = (float)L::w(q);
+        if (qb == q) {
+            drho = fma2(pack2(w, w), g[q], drho);
+            continue;
+        }
+        const int i = pair_leads<L>(q) ? q : qb;
+        drho = fma2(pack2(w, w), s[i], drho);
+        const int c[3] = {L::cx(i), L::cy(i), L::cz(i)};
+#pragma unroll
+        for (int m = 0; m < L::D; ++m)
+            if (c[m] != 0) j[m] = fma2(c[m] > 0 ? pack2(w, w) : pack2(-w, -w), d[i], j[m]);
+    }
+    const f32x2 r = fma2(drho, pack2(k.invS), pack2(k.rho0));
+    rho[0] = low2(r);
+    rho[1] = high2(r);
+#pragma unroll
+    for (int m = 0; m < L::D; ++m) j[m] = fma2(j[m], pack2(k.invS), pack2(k.hF[m]));
+    // findFluidVelocity: u = 0 where rho == 0
+    const f32x2 inv = pack2(rho[0] != 0.f ? recip(rho[0]) : 0.f, rho[1] != 0.f ? recip(rho[1]) : 0.f);
+    f32x2 u[3];
+#pragma unroll
+    for (int m = 0; m < L::D; ++m) u[m] = mul2(j[m], inv);
+    // sums of products in the order the scalar code's are contracted
+    f32x2 usq = fma2(u[0], u[0], mul2(u[1], u[1])), uF = fma2(u[0], pack2(k.F[0]), mul2(u[1], pack2(k.F[1])));
+    if (L::D == 3) {
+        usq = fma2(u[2], u[2], usq);
+        uF = fma2(u[2], pack2(k.F[2]), uF);
+    }
+    const f32x2 Srq = mul2(pack2(k.S), a.incompressible ? pack2(k.rho_inc) : r);
+    const f32x2 E0 = fma2(mul2(pack2(-1.5f, -1.5f), Srq), usq, drho);
+    const f32x2 e0 = fma2(pack2(k.omE), E0, mul2(pack2(k.gK0), uF));
+    const f32x2 k45 = mul2(pack2(k.c45), Srq), k3 = mul2(pack2(k.c3), Srq);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int qb = L::opp(q);
+        if (qb < q) continue;
+        if (qb == q) {
+            g[q] = fma2(pack2(k.rest), g[q], e0);
+            continue;
+        }
+        const int i = pair_leads<L>(q) ? q : qb, ib = L::opp(i);
+        const int c[3] = {L::cx(i), L::cy(i), L::cz(i)};
+        f32x2 cu = 0;
+        bool any = false;
+#pragma unroll
+        for (int m = 0; m < L::D; ++m)
+            if (c[m] != 0) {
+                cu = !any ? u[m] : (c[m] > 0 ? add2(cu, u[m]) : sub2(cu, u[m]));
+                any = true;
+            }
+        const f32x2 E = fma2(fma2(k45, cu, pack2(k.gB[i])), cu, e0);
+        const f32x2 O = fma2(k3, cu, pack2(k.gA[i]));
+        if (TRT) {
+            const f32x2 es = fma2(pack2(k.le), s[i], E), od = fma2(pack2(k.lo), d[i], O);
+            g[i] = add2(es, od);
+            g[ib] = sub2(es, od);
+        } else {
+            g[i] = fma2(pack2(k.hsum), g[i], add2(E, O));
+            g[ib] = fma2(pack2(k.hsum), g[ib], sub2(E, O));
+        }
+    }
+}
+
 template <class L, int ST, bool TRT>
 struct NodeState {
     using R = typename Store<ST>::R;
@@ -540,8 +705,13 @@ template <> struct Vec4<ST_F32> {
         v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
     }
     static __device__ __forceinline__ void load(const void* base, int cell0, float* v) {
-        unpack(__ldcs(reinterpret_cast<const float4*>(static_cast<const float*>(base) + cell0)), v);
+        unpack(load_raw(base, cell0), v);
     }
+    static __device__ __forceinline__ raw load_raw(const void* base, int cell0) {
+        return __ldcs(reinterpret_cast<const float4*>(static_cast<const float*>(base) + cell0));
+    }
+    // the values of cells (0, 1) (h = 0) or (2, 3)
+    static __device__ __forceinline__ f32x2 two(const raw& q, int h) { return h ? pack2(q.z, q.w) : pack2(q.x, q.y); }
     // values of direction `dir` for cells cell0 .. cell0+3 (cell0 a multiple of 4)
     static __device__ __forceinline__ void store(void* base, int cell0, int, float a0, float a1, float a2, float a3,
                                                  const unsigned*, bool keep = false) {
@@ -566,6 +736,10 @@ template <> struct Vec4<ST_F16> {
     }
     static __device__ __forceinline__ raw load_raw(const void* base, int cell0) {
         return __ldcs(reinterpret_cast<const uint2*>(static_cast<const __half*>(base) + cell0));
+    }
+    static __device__ __forceinline__ f32x2 two(const raw& q, int h) {
+        const unsigned w = h ? q.y : q.x;
+        return pack2(__half22float2(*reinterpret_cast<const __half2*>(&w)));
     }
     // value `hi` (0: low half, 1: high half) of a packed pair
     static __device__ __forceinline__ float lane(unsigned w, int hi) {
@@ -615,6 +789,10 @@ template <> struct Vec4<ST_BF16> {
     static __device__ __forceinline__ raw load_raw(const void* base, int cell0) {
         return __ldcs(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(base) + cell0));
     }
+    static __device__ __forceinline__ f32x2 two(const raw& q, int h) {
+        const unsigned w = h ? q.y : q.x;
+        return pack2(__bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)));
+    }
     static __device__ __forceinline__ float lane(unsigned w, int hi) {
         const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
         return hi ? f.y : f.x;
@@ -662,11 +840,12 @@ constexpr int x_slot(int i) {  // exchange slot of direction i (cx != 0)
 
 // The pushes of one thread's four x-nodes (x0 .. x0+3 of row (y, z)) after
 // their collision: direction i goes to x + c_i with aligned vector stores.
+// g(k, i) is node x0 + k's value of direction i;
 // from_left(i) / from_right(i) give the value of the +x / -x moving direction
 // i that the neighbouring segment pushes into this one (read next to the
 // store that needs it, so that the exchanged values are not all live at once).
-template <class L, int ST, class FromLeft, class FromRight>
-__device__ __forceinline__ void bulk_v4_push(const StepArgs& a, const float (&g)[4][L::Q], FromLeft from_left,
+template <class L, int ST, class Own, class FromLeft, class FromRight>
+__device__ __forceinline__ void bulk_v4_push(const StepArgs& a, Own g, FromLeft from_left,
                                              FromRight from_right, int x0, int y, int z, const unsigned* dither,
                                              bool keep = false) {
     constexpr int Q = L::Q;
@@ -677,11 +856,11 @@ __device__ __forceinline__ void bulk_v4_push(const StepArgs& a, const float (&g)
     for (int i = 0; i < Q; ++i) {
         const int t0 = x0 + nx * (ys[L::cy(i) + 1] + ny * zs[L::cz(i) + 1]);
         if (L::cx(i) == 0) {
-            Vec4<ST>::store(a.dstq[i], t0, i, g[0][i], g[1][i], g[2][i], g[3][i], dither, keep);
+            Vec4<ST>::store(a.dstq[i], t0, i, g(0, i), g(1, i), g(2, i), g(3, i), dither, keep);
         } else if (L::cx(i) == 1) {
-            Vec4<ST>::store(a.dstq[i], t0, i, from_left(i), g[0][i], g[1][i], g[2][i], dither, keep);
+            Vec4<ST>::store(a.dstq[i], t0, i, from_left(i), g(0, i), g(1, i), g(2, i), dither, keep);
         } else {
-            Vec4<ST>::store(a.dstq[i], t0, i, g[1][i], g[2][i], g[3][i], from_right(i), dither, keep);
+            Vec4<ST>::store(a.dstq[i], t0, i, g(1, i), g(2, i), g(3, i), from_right(i), dither, keep);
         }
     }
 }
@@ -695,7 +874,11 @@ __device__ __forceinline__ void bulk_v4_push(const StepArgs& a, const float (&g)
 // Threads past the tile's rows only take part in the barrier.
 // SR: the 2-byte stores round stochastically (a separate instantiation, so
 // that the nearest-rounding kernels keep their register allocation)
-template <class L, int ST, bool TRT, int B, bool SR = false>
+// X2: the packed collision (collide_x2).  It wants its constants doubled, which
+// the kernel's own parameters hold; the queue and batch kernels read a
+// replica's arguments from global memory, where the packed form is slower
+// (512 D2Q9 replicas' tiles 62 -> 92 us per tick) and the scalar one stays.
+template <class L, int ST, bool TRT, int B, bool SR = false, bool X2 = false>
 __device__ __forceinline__ void bulk_v4_tile(const StepArgs& a, long long tile, float (*s_ex)[B],
                                              bool keep = false) {
     using R = float;
@@ -711,59 +894,94 @@ __device__ __forceinline__ void bulk_v4_tile(const StepArgs& a, long long tile, 
     const bool valid = row < a.vrows && y < ny;
     const int x0 = 4 * j;
     const int cell0 = valid ? x0 + nx * (y + ny * z) : 0;
-    R g[4][Q];
-    const R Fx = a.kf.F[0], Fy = a.kf.F[1], Fz = a.kf.F[2];
+    f32x2 g[2][X2 ? Q : 1];  // X2: nodes (x0, x0 + 1) and (x0 + 2, x0 + 3)
+    R gs[4][X2 ? 1 : Q];     // else the four nodes
     bool bad = false;
-    if constexpr (TRT && Store<ST>::bytes == 2) {
-        // 2-byte TRT: the pair sums and differences take the first value of
-        // each pair straight from its 16-bit form (Vec4::sum_diff).  The
-        // threads past the tile's rows load cells 0..3 (cell0 = 0, in bounds)
-        // and store nothing.  128^3 FP16 pass: 6.6 % fewer instructions than
-        // converting every value first, bit-identical results.
+    if constexpr (X2) {
+        // The threads past the tile's rows load cells 0..3 (cell0 = 0, in bounds)
+        // and store nothing.
         typename Vec4<ST>::raw q[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i) q[i] = Vec4<ST>::load_raw(a.srcq[i], cell0);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            R s[Q], d[Q];
+        for (int h = 0; h < 2; ++h) {
+            f32x2 s[Q], d[Q];
+            float rho[2];
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
                 const int ib = L::opp(i);
-                if (ib < i) continue;
-                const unsigned wa = k < 2 ? q[i].x : q[i].y;  // cells (0, 1) | (2, 3)
                 if (ib == i) {
-                    g[k][i] = Vec4<ST>::lane(wa, k & 1);
-                    continue;
+                    g[h][i] = Vec4<ST>::two(q[i], h);
+                } else if (pair_leads<L>(i)) {
+                    const f32x2 ga = Vec4<ST>::two(q[i], h), gb = Vec4<ST>::two(q[ib], h);
+                    s[i] = add2(ga, gb);
+                    d[i] = sub2(ga, gb);
+                    if (!TRT) {
+                        g[h][i] = ga;
+                        g[h][ib] = gb;
+                    }
                 }
-                const R b = Vec4<ST>::lane(k < 2 ? q[ib].x : q[ib].y, k & 1);
-                Vec4<ST>::sum_diff(wa, k & 1, b, s[i], d[i]);
             }
-            bad |= bad_density(collide_sd<L, R, TRT>(a, g[k], s, d, Fx, Fy, Fz, false));
+            collide_x2<L, TRT>(a, g[h], s, d, rho);
+            bad |= bad_density(rho[0]) || bad_density(rho[1]);
         }
     } else {
+        const R Fx = a.kf.F[0], Fy = a.kf.F[1], Fz = a.kf.F[2];
+        if constexpr (TRT && Store<ST>::bytes == 2) {
+            // 2-byte TRT: the pair sums and differences take the first value of
+            // each pair straight from its 16-bit form (Vec4::sum_diff).  The
+            // threads past the tile's rows load cells 0..3 (cell0 = 0, in bounds)
+            // and store nothing.  128^3 FP16 pass: 6.6 % fewer instructions than
+            // converting every value first, bit-identical results.
+            typename Vec4<ST>::raw q[Q];
 #pragma unroll
-        for (int i = 0; i < Q; ++i) {
-            R v[4] = {0, 0, 0, 0};
-            if (valid) Vec4<ST>::load(a.srcq[i], cell0, v);
-            g[0][i] = v[0];
-            g[1][i] = v[1];
-            g[2][i] = v[2];
-            g[3][i] = v[3];
+            for (int i = 0; i < Q; ++i) q[i] = Vec4<ST>::load_raw(a.srcq[i], cell0);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                R s[Q], d[Q];
+#pragma unroll
+                for (int i = 0; i < Q; ++i) {
+                    const int ib = L::opp(i);
+                    if (ib < i) continue;
+                    const unsigned wa = k < 2 ? q[i].x : q[i].y;  // cells (0, 1) | (2, 3)
+                    if (ib == i) {
+                        gs[k][i] = Vec4<ST>::lane(wa, k & 1);
+                        continue;
+                    }
+                    const R b = Vec4<ST>::lane(k < 2 ? q[ib].x : q[ib].y, k & 1);
+                    Vec4<ST>::sum_diff(wa, k & 1, b, s[i], d[i]);
+                }
+                bad |= bad_density(collide_sd<L, R, TRT>(a, gs[k], s, d, Fx, Fy, Fz, false));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                R v[4] = {0, 0, 0, 0};
+                if (valid) Vec4<ST>::load(a.srcq[i], cell0, v);
+                gs[0][i] = v[0];
+                gs[1][i] = v[1];
+                gs[2][i] = v[2];
+                gs[3][i] = v[3];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) bad |= bad_density(collide<L, R, TRT>(a, gs[k], Fx, Fy, Fz, false));
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) bad |= bad_density(collide<L, R, TRT>(a, g[k], Fx, Fy, Fz, false));
     }
     report_density(valid && bad, a.err);
+    auto own = [&](int k, int i) {
+        if constexpr (X2) return k & 1 ? high2(g[k >> 1][i]) : low2(g[k >> 1][i]);
+        else return gs[k][i];
+    };
     constexpr bool sr = SR && Store<ST>::bytes == 2;
     unsigned dw[4];
-    if (sr) rs_words(group_dither(cell0, g[0][1], g[0][2], g[0][3]), dw);
+    if (sr) rs_words(group_dither(cell0, own(0, 1), own(0, 2), own(0, 3)), dw);
     const unsigned* dither = sr ? dw : nullptr;
     // the value of each +-x direction that leaves this thread's 4-node segment
     if (row < a.vrows) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
-            if (L::cx(i) == 1) s_ex[x_slot<L>(i)][tid] = g[3][i];
-            if (L::cx(i) == -1) s_ex[x_slot<L>(i)][tid] = g[0][i];
+            if (L::cx(i) == 1) s_ex[x_slot<L>(i)][tid] = own(3, i);
+            if (L::cx(i) == -1) s_ex[x_slot<L>(i)][tid] = own(0, i);
         }
     }
     __syncthreads();
@@ -771,24 +989,23 @@ __device__ __forceinline__ void bulk_v4_tile(const StepArgs& a, long long tile, 
     const int left = row * RT + (j == 0 ? RT - 1 : j - 1);
     const int right = row * RT + (j == RT - 1 ? 0 : j + 1);
     bulk_v4_push<L, ST>(
-        a, g, [&](int i) { return s_ex[x_slot<L>(i)][left]; }, [&](int i) { return s_ex[x_slot<L>(i)][right]; }, x0,
+        a, own, [&](int i) { return s_ex[x_slot<L>(i)][left]; }, [&](int i) { return s_ex[x_slot<L>(i)][right]; }, x0,
         y, z, dither, keep);
 }
 
 // Resident threads per SM the vector bulk kernels are compiled for: a D2Q9
-// thread holds 36 populations and fits 64 registers (32 warps per SM); the
-// 3D sets take up to 128 (16 warps per SM) with FP32/FP64 storage, which is
-// memory-bound, and up to 96 (20 warps per SM) with 2-byte storage, whose
-// conversions make it issue-bound as well: the extra warps took its 128^3
-// pass from 28.4 to 26.9 us, with no change for FP32.
-// Stochastic rounding (one conversion per two values with the group's
-// random words) fits the same 96 registers.  A D3Q27 thread holds 108
-// populations: 12 warps per SM (168 registers) with FP32/FP64 storage, 14
-// (144) with 2-byte storage, so that neither spills.
-template <class L, int ST = ST_F32, bool SR = false>
+// thread holds 36 populations and fits 64 registers (32 warps per SM).  The 3D
+// sets hold 60 to 108 and must not spill: with the packed collision D3Q15 and
+// D3Q19 take 128 registers (16 warps), D3Q15 with 2-byte storage 96 (20 warps),
+// D3Q27 168 (12 warps).  D3Q19 FP16 compiled for 20 warps spilled 44 bytes per
+// thread and its 128^3 pass took 35.9 us instead of 28.7.  The scalar
+// collision (X2 = false) fits 20 warps with 2-byte storage (14 for D3Q27).
+template <class L, int ST = ST_F32, bool SR = false, bool X2 = false>
 constexpr int bulk_threads_per_sm() {
-    return L::Q <= 9 ? 1024
-                     : (L::Q > 19 ? (Store<ST>::bytes == 2 ? 448 : 384) : (Store<ST>::bytes == 2 ? 640 : 512));
+    if (L::Q <= 9) return 1024;
+    if (Store<ST>::bytes != 2) return L::Q > 19 ? 384 : 512;
+    if (X2) return L::Q > 19 ? 384 : (L::Q == 19 ? 512 : 640);
+    return L::Q > 19 ? 448 : 640;
 }
 
 // the vector bulk pass over all tiles, one CTA of B threads per tile
@@ -799,7 +1016,7 @@ constexpr int bulk_threads_per_sm() {
 // instead of HBM (the 128^3 FP32 tick 55.2 -> 51.3 us).  The result does not
 // depend on the order.
 template <class L, int ST, bool TRT, int B, bool SR>
-__global__ void __launch_bounds__(B, bulk_threads_per_sm<L, ST, SR>() / B) k_bulk_v4(const StepArgs a) {
+__global__ void __launch_bounds__(B, bulk_threads_per_sm<L, ST, SR, true>() / B) k_bulk_v4(const StepArgs a) {
     __shared__ float s_ex[x_moving_dirs<L>()][B];
     grid_dep_trigger();  // the fix-up may start its stores-free part during the last wave
     const long long tiles = (long long)a.vnt1 * a.g.n[2];
@@ -808,7 +1025,7 @@ __global__ void __launch_bounds__(B, bulk_threads_per_sm<L, ST, SR>() / B) k_bul
     // none, 50.5 with two fifths, 49.4 with three, 50.2 with four, 51.6 with
     // all); the issue-bound 2-byte passes measured slower with it
     const bool keep = Store<ST>::bytes == 4 && (long long)blockIdx.x * 5 >= tiles * 2;
-    bulk_v4_tile<L, ST, TRT, B, SR>(a, a.reverse ? tiles - 1 - (long long)blockIdx.x : (long long)blockIdx.x, s_ex,
+    bulk_v4_tile<L, ST, TRT, B, SR, true>(a, a.reverse ? tiles - 1 - (long long)blockIdx.x : (long long)blockIdx.x, s_ex,
                                     keep);
 }
 
