@@ -140,10 +140,16 @@ struct StepArgs {
     int vrows;                            // x-rows per tile of the vector bulk pass
     long long vtiles;                     // tiles of the vector bulk pass
     int vnt1;                             // vector tiles per z-slice
-    int pad;
+    int walkctas, listctas;               // CTAs per particle of k_fixup_walk, behind and beside the bulk pass
     const int* nbox;                      // [nparts][6] solid boxes (lo, hi) the fix-up of this tick uses
     const unsigned char* vnear;           // [vtiles] tiles next to wall links (static) or null
     double* partial;
+    // link slots computed beside the bulk pass and stored after it (fixup.cuh):
+    // the slot's index in dst, its value, and {slots listed, k_fixup_store CTAs that have read that}
+    long long* slot_at;
+    void* slot_val;
+    int* slot_n;
+    int slot_cap;
     int* err;
     double rho0;                          // shift density of the stored populations
     double scale, inv_scale;              // storage scale (F16/BF16)

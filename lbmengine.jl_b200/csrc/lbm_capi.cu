@@ -86,7 +86,7 @@ struct lbm_handle {
     Ops ops{};
     // device state: the main stream and a side stream for the particle update
     cudaStream_t stream = nullptr, side = nullptr;
-    cudaEvent_t ev_fix = nullptr, ev_part = nullptr;
+    cudaEvent_t ev_fix = nullptr, ev_part = nullptr, ev_list = nullptr;
     bool part_pending = false;
     // vector bulk pass: tiles of vrows full x-rows, vblock threads per tile
     int vrows = 0, vnt1 = 0, vblock = 0;
@@ -110,6 +110,11 @@ struct lbm_handle {
     TickCounters* d_tq = nullptr;
     long long spin_limit = kSpinLimit;  // polls before a wait of the tick kernel gives up
     int wait_extra = 0;                 // test knob: added to the fix-up items' wait target
+    // the fix-up beside the bulk pass: the list of link slots (fixup.cuh)
+    long long* d_slot_at = nullptr;
+    void* d_slot_val = nullptr;
+    int* d_slot_n = nullptr;
+    int slot_cap = 0;
     // many ticks per launch (resident.cuh)
     bool auto_schedule = false;         // the caller left the schedule to the library
     int res_ctas = -1;                  // CTAs of the launch; 0: does not apply, -1: not looked up yet
@@ -519,6 +524,33 @@ void lattice_vectors(int lattice, int* cx, int* cy, int* cz, int* q) {
     }
 }
 
+// chunks of the link list of the largest particle, about: a sphere has 1.55
+// link nodes per unit of its surface
+int list_chunks(const lbm_handle* h) {
+    double r = 0;
+    for (const auto& P : h->hparts) r = std::max(r, P.radius / h->dx);
+    const double entries = 1.55 * M_PI * (h->dims == 3 ? 4.0 * r * r : 2.0 * r);
+    return (int)std::min(std::ceil(entries / kFixBlock), (double)std::max(1, h->maxchunks));
+}
+
+// the bulk pass's bytes at 6.5 TB/s, in us
+double bulk_us(const lbm_handle* h) { return 2.0 * h->q * storage_bytes(h->storage) * (double)h->N / 6.5e6; }
+
+// CTAs per particle of the fix-up beside the bulk pass.  A CTA takes up to
+// 20 us per chunk and the particle update behind it about 30: up to four
+// chunks in turn where the bulk pass hides both, because more CTAs at once
+// only take registers from it (64 particles of r = 6 in 192^3 BF16:
+// 3 / 4 / 6 / 18 CTAs per particle 107.1 / 106.5 / 107.4 / 110.8 us per tick; 32 of r = 8 in 128^3 FP32: 6 / 19 CTAs 92.8 / 59.7 us).
+int list_ctas(const lbm_handle* h) {
+    const int turns = (int)std::min(4.0, std::max(1.0, std::floor((bulk_us(h) - 30.0) / 20.0)));
+    return (list_chunks(h) + turns - 1) / turns;
+}
+
+// CTAs per particle of k_fixup_walk
+int walk_ctas(const lbm_handle* h) {
+    return std::min(h->maxchunks, std::max(kFixCtasPerPart, list_chunks(h)));
+}
+
 // Kernel arguments of one tick from buffer `src`, with the fix-up's
 // momentum-exchange partials in `partial`.  Uses no host heap.
 StepArgs make_step_args(const lbm_handle* h, int src, double* partial) {
@@ -552,6 +584,12 @@ StepArgs make_step_args(const lbm_handle* h, int src, double* partial) {
     a.nbox = h->d_nbox[src];
     a.vnear = h->d_vnear;
     a.partial = partial;
+    a.slot_at = h->d_slot_at;
+    a.slot_val = h->d_slot_val;
+    a.slot_n = h->d_slot_n;
+    a.slot_cap = h->slot_cap;
+    a.listctas = list_ctas(h);
+    a.walkctas = walk_ctas(h);
     a.err = h->d_err;
     a.rho0 = h->rho0;
     a.scale = h->scale;
@@ -737,9 +775,73 @@ bool fixup_walk(const lbm_handle* h) { return (long long)h->hparts.size() * h->m
 // CTAs of a fix-up launch
 long long fixup_grid(const lbm_handle* h) {
     if (!fixup_walk(h)) return fixup_blocks(h);
-    return (long long)h->hparts.size() * fixup_ctas_per_particle(h->maxchunks) +
+    return (long long)h->hparts.size() * walk_ctas(h) +
            (h->nwlinks + kFixBlock - 1) / kFixBlock + (h->nwnodes + kFixBlock - 1) / kFixBlock;
 }
+
+// The link slots a model can have.  A particle's solid nodes on a lattice line
+// along c_j are contiguous (a sphere is convex), so direction j has at most
+// one link per line that meets the sphere: |c_j| lines per unit area (length
+// in 2D) across c_j, in the projected sphere grown by 1.5 nodes.  A wall-link
+// entry has at most Q - 1.
+long long slot_bound(const lbm_handle* h) {
+    int cx[27], cy[27], cz[27], q = 0;
+    lattice_vectors(h->lattice, cx, cy, cz, &q);
+    long long n = (long long)h->nwlinks * (q - 1);
+    for (const auto& P : h->hparts) {
+        const double r = P.radius / h->dx + 1.5;
+        double m = 0;
+        for (int i = 1; i < q; ++i) {
+            const double c = std::sqrt((double)(cx[i] * cx[i] + cy[i] * cy[i] + cz[i] * cz[i]));
+            m += std::ceil(c * (h->dims == 2 ? 2.0 * r : M_PI * r * r)) + 1;
+        }
+        n += (long long)std::min(m, (double)P.link_cap * (q - 1));
+    }
+    return n;
+}
+
+// The list of link slots, sized for the model's particles; without the memory
+// (or past 2^30 slots) the fix-up stays behind the bulk pass (slot_cap 0).
+int slot_list(lbm_handle* h) {
+    const long long n = slot_bound(h);
+    if (n <= h->slot_cap || n >= (1LL << 30)) return LBM_OK;
+    dev_free(h->d_slot_at);
+    dev_free(h->d_slot_val);
+    h->slot_cap = 0;
+    if (block_alloc((void**)&h->d_slot_at, sizeof(long long) * n) != cudaSuccess ||
+        block_alloc((void**)&h->d_slot_val, (size_t)storage_bytes(h->storage) * n) != cudaSuccess ||
+        (!h->d_slot_n && block_alloc((void**)&h->d_slot_n, 2 * sizeof(int)) != cudaSuccess)) {
+        cudaGetLastError();
+        return LBM_OK;
+    }
+    CUDA_TRY(h, cudaMemsetAsync(h->d_slot_n, 0, 2 * sizeof(int), h->stream));
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));  // a batch launches on its own streams
+    h->slot_cap = (int)n;
+    return LBM_OK;
+}
+
+// Whether the fix-up runs beside the bulk pass.  Behind it, it adds its own
+// time, one wave of k_fixup_walk (296 CTAs) after another; beside it, the chain
+// fix-up -> particle update has to fit into the bulk pass, and a launch is
+// added.  So: more chunks than one wave, and a bulk pass (its bytes at 6.5 TB/s)
+// no shorter than the particle update (18 us + 0.095 us r^2 in 3D, 10 us in
+// 2D), or many waves of small particles.  Ticks in us, behind / beside:
+//   D3Q19  192^3 BF16, 64 of r = 6 125 / 107;  27 of r = 6 111 / 100
+//          128^3 FP32, 8 of r = 8 (152 chunks) 57.1 / 57.8;  16 66.6 / 64.4;  32 76.7 / 60.0;
+//                      8 of r = 16 77.7 / 69.4;  1 of r = 20 (122 chunks) 61.8 / 66.5;  1 of r = 32 101 / 103
+//          256^3 FP32, 4 of r = 32 432 / 406;  FP16, 27 of r = 20 318 / 279
+//          192^3 FP32, 1 of r = 40 228 / 242;  96^3 FP32, 27 of r = 6 35.7 / 36.8
+//          64^3  FP32, 64 of r = 6 (704 chunks) 44.7 / 37.4;  64 of r = 4 (320 chunks) 25.7 / 30.4
+//   D2Q9   2048^2 FP32, 250 of r = 20 103 / 66;  1024^2 FP32, 250 of r = 8 28.5 / 23.5
+constexpr long long kFixWave = 296;
+bool many_chunks(const lbm_handle* h) {
+    const long long np = (long long)h->hparts.size(), chunks = np * list_chunks(h);
+    if (!fixup_walk(h) || chunks <= kFixWave) return false;
+    double r = 0;
+    for (const auto& P : h->hparts) r = std::max(r, P.radius / h->dx);
+    return bulk_us(h) >= (h->dims == 3 ? 18.0 + 0.095 * r * r : 10.0) || (chunks >= 2 * kFixWave && np >= 8);
+}
+bool fixup_beside(const lbm_handle* h) { return h->profiling < 2 && h->slot_cap > 0 && many_chunks(h); }
 
 // the persistent tick kernel applies to the vector bulk kernel with
 // kTickBlock-thread tiles, when there is boundary work to overlap
@@ -996,7 +1098,7 @@ int resident_ticks(lbm_handle* h, int64_t nsteps, int64_t* ran) {
 int launches_per_tick(const lbm_handle* h) {
     if (use_tick_kernel(h)) return 1;
     const bool fix = fixup_blocks(h) > 0;
-    return 1 + (fix ? 1 : 0) + (h->hparts.empty() ? 0 : 1);  // the particle update rebuilds its links itself
+    return 1 + (fixup_beside(h) ? 2 : fix ? 1 : 0) + (h->hparts.empty() ? 0 : 1);  // the particle update rebuilds its links itself
 }
 
 // events of graph slot s: [0] before bulk, [1] after bulk, [2] after fix-up, [3] after particles
@@ -1044,12 +1146,26 @@ void programmatic_from(cudaStream_t s, cudaGraphNode_t from) {
     cudaStreamUpdateCaptureDependencies_v2(s, nodes, edges, n, cudaStreamSetCaptureDependencies);
 }
 
+// the particle update of a tick on the side stream
+void enqueue_particles(lbm_handle* h, int src, int slot) {
+    ParticleArgs pa = particle_args(h, 0, 0, src);
+    pa.inline_links = 1;
+    launch_interactions(h, h->side);
+    h->ops.particles(pa, (unsigned)h->hparts.size(), h->side);
+    prof_record(h, slot, 3, h->side);
+    cudaEventRecord(h->ev_part, h->side);
+    h->part_pending = true;
+}
+
 // Enqueue one tick (capturable); `slot` selects the profiling events.
 // Persistent tick kernel: one launch.  Otherwise
 //   main: bulk(n) -> [wait particles(n-1)] -> fixup(n) -> bulk(n+1) ...
 //   side:                    particles(n) after fixup(n)
 // The bulk pass never reads particle state, so the particle update of tick n
-// runs concurrently with the bulk pass of tick n+1.
+// runs concurrently with the bulk pass of tick n+1.  With many particles
+// (fixup_beside) the fix-up does too:
+//   main: bulk(n) -> [wait list(n)] -> store(n) -> bulk(n+1) ...
+//   side: [wait store(n-1)] -> list(n) -> particles(n)
 void enqueue_tick(lbm_handle* h, int src, int slot) {
     prof_record(h, slot, 0, h->stream);
     if (use_tick_kernel(h)) {
@@ -1059,6 +1175,14 @@ void enqueue_tick(lbm_handle* h, int src, int slot) {
         return;
     }
     const StepArgs a = step_args(h, src);
+    const bool beside = fixup_beside(h);
+    if (beside) {
+        cudaEventRecord(h->ev_fix, h->stream);
+        cudaStreamWaitEvent(h->side, h->ev_fix, 0);
+        h->ops.fixup_list(a, (unsigned)(a.nparts * a.listctas + (a.nwlinks + kFixBlock - 1) / kFixBlock), h->side);
+        cudaEventRecord(h->ev_list, h->side);
+        enqueue_particles(h, src, slot);
+    }
     launch_bulk(h, a, h->stream);
     prof_record(h, slot, 1, h->stream);
     // The fix-up follows the bulk pass through a programmatic edge (it computes
@@ -1069,6 +1193,12 @@ void enqueue_tick(lbm_handle* h, int src, int slot) {
     const bool early = h->profiling < 2;
     const cudaGraphNode_t bulk_node = early ? capture_tail(h->stream) : nullptr;
     bool waited = false;
+    if (beside) {
+        cudaStreamWaitEvent(h->stream, h->ev_list, 0);
+        if (bulk_node) programmatic_from(h->stream, bulk_node);
+        h->ops.fixup_store(a, h->stream, false);
+        return;
+    }
     if (h->part_pending) {
         cudaStreamWaitEvent(h->stream, h->ev_part, 0);
         h->part_pending = false;
@@ -1084,13 +1214,7 @@ void enqueue_tick(lbm_handle* h, int src, int slot) {
         cudaEventRecord(h->ev_fix, h->stream);
         cudaStreamWaitEvent(h->side, h->ev_fix, 0);
         prof_record(h, slot, 2, h->side);
-        ParticleArgs pa = particle_args(h, 0, 0, src);
-        pa.inline_links = 1;
-        launch_interactions(h, h->side);
-        h->ops.particles(pa, (unsigned)a.nparts, h->side);
-        prof_record(h, slot, 3, h->side);
-        cudaEventRecord(h->ev_part, h->side);
-        h->part_pending = true;
+        enqueue_particles(h, src, slot);
     }
 }
 
@@ -1118,7 +1242,9 @@ int build_graph(lbm_handle* h, int start, int size_idx) {
         cudaGetLastError();
         return set_err(h, LBM_ERR_CUDA, std::string("graph capture failed: ") + cudaGetErrorString(e));
     }
-    e = cudaGraphInstantiate(&gr.exec, graph, 0);
+    // with the nodes' priorities: the side stream's CTAs are placed before those
+    // the bulk pass still has waiting (else they start as it ends)
+    e = cudaGraphInstantiate(&gr.exec, graph, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
         gr.exec = nullptr;
@@ -1259,6 +1385,9 @@ void destroy_all(lbm_handle* h) {
     dev_free(h->d_dmap);
     dev_free(h->d_targs);
     dev_free(h->d_rjobs);
+    dev_free(h->d_slot_at);
+    dev_free(h->d_slot_val);
+    dev_free(h->d_slot_n);
     dev_free(h->d_pmask);
     dev_free(h->d_wmask);
     dev_free(h->d_rsync);
@@ -1270,6 +1399,7 @@ void destroy_all(lbm_handle* h) {
     if (h->t_end) cudaEventDestroy(h->t_end);
     if (h->ev_fix) cudaEventDestroy(h->ev_fix);
     if (h->ev_part) cudaEventDestroy(h->ev_part);
+    if (h->ev_list) cudaEventDestroy(h->ev_list);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
@@ -1623,7 +1753,8 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
                 ? LBM_OK : set_err(h, LBM_ERR_CUDA, "stream creation failed"));
     }
     TRY(cudaEventCreateWithFlags(&h->ev_fix, cudaEventDisableTiming) == cudaSuccess &&
-                cudaEventCreateWithFlags(&h->ev_part, cudaEventDisableTiming) == cudaSuccess
+                cudaEventCreateWithFlags(&h->ev_part, cudaEventDisableTiming) == cudaSuccess &&
+                cudaEventCreateWithFlags(&h->ev_list, cudaEventDisableTiming) == cudaSuccess
             ? LBM_OK : set_err(h, LBM_ERR_CUDA, "event creation failed"));
     TRY(dev_alloc(h, &h->d_tq, sizeof(TickCounters)));
     if (cudaMemsetAsync(h->d_tq, 0, sizeof(TickCounters), h->stream) != cudaSuccess)
@@ -1871,7 +2002,8 @@ int lbm_step(lbm_handle* h, int64_t nsteps) {
     BIND(h);
     const bool resident = use_resident(h);
     if (!resident) {
-        const int rc = prepare_tick(h);
+        int rc = prepare_tick(h);
+        if (!rc && many_chunks(h) && !use_tick_kernel(h)) rc = slot_list(h);
         if (rc) return rc;
     }
     const bool direct = h->calls++ == 0 && nsteps <= kFirstCallDirectTicks && !resident;
@@ -2647,7 +2779,7 @@ struct lbm_batch {
     std::vector<lbm_handle*> reps;
     Ops ops{};
     cudaStream_t stream = nullptr, side = nullptr;
-    cudaEvent_t ev_fix = nullptr, ev_part = nullptr;
+    cudaEvent_t ev_fix = nullptr, ev_part = nullptr, ev_list = nullptr;
     bool part_pending = false;
     int sms = 0, max_per_sm = 0;
     lbm_batch_tuning tuning{};
@@ -2658,6 +2790,7 @@ struct lbm_batch {
     int4* d_amap = nullptr;
     int2 *d_bmap = nullptr, *d_cmap = nullptr, *d_dmap = nullptr;
     long long na = 0, nb = 0, nc = 0, nd = 0;
+    unsigned slot_ctas = 0;  // k_fixup_store_batch CTAs per replica; 0: the fix-up follows the tiles
     StepArgs* d_targs = nullptr;      // [2][n]
     ParticleArgs* d_pargs = nullptr;  // [2][n]
     TickCounters* d_tq = nullptr;     // [0] main-stream launches, [1] side-stream launches
@@ -2744,6 +2877,8 @@ int batch_prepare(lbm_batch* b) {
         for (long long k = 0; k < nfb; ++k) bm.push_back(make_int2(r, (int)k));
         for (int p = 0; p < np; ++p) cm.push_back(make_int2(r, p));
         maxt = std::max(maxt, h->vtiles);
+        const int rc = slot_list(h);
+        if (rc) return bset_err(b, rc, h->err);
     }
     if (b->tuning.tile_order == 1) {
         for (long long t = 0; t < maxt; ++t)
@@ -2788,6 +2923,14 @@ int batch_prepare(lbm_batch* b) {
     b->nb = (long long)bm.size();
     b->nc = (long long)cm.size();
     b->nd = (long long)dm.size();
+    // the fix-up beside the tiles: where every replica has its list, and there are particles
+    int cap = 0;
+    bool lists = b->nb > 0 && b->nc > 0 && n <= 65535;
+    for (const lbm_handle* h : b->reps) {
+        cap = std::max(cap, h->slot_cap);
+        lists = lists && (h->slot_cap > 0 || fixup_blocks(h) == 0);
+    }
+    b->slot_ctas = lists ? fixup_store_ctas(cap) : 0;
     b->ready = true;
     return LBM_OK;
 }
@@ -2819,6 +2962,13 @@ void batch_launch(lbm_batch* b, int s, const TickItems& it, int q, cudaStream_t 
                 b->d_err + n, grid, st, b->reps[0]->rounding == LBM_ROUND_STOCHASTIC);
 }
 
+// the particle updates of a tick on the side stream
+void batch_particles(lbm_batch* b, int s) {
+    batch_launch(b, s, batch_items(b, false, false, true, false, 0), 1, b->side);
+    cudaEventRecord(b->ev_part, b->side);
+    b->part_pending = true;
+}
+
 // one tick of every replica with arguments of parity s (capturable)
 void batch_enqueue(lbm_batch* b, int s) {
     if (b->tuning.schedule == LBM_SCHEDULE_PERSISTENT) {
@@ -2826,12 +2976,27 @@ void batch_enqueue(lbm_batch* b, int s) {
         return;
     }
     // stream order: all tiles; then the fix-up blocks once the previous
-    // particle update is done; the particle update on the side stream
+    // particle update is done; the particle update on the side stream.  With
+    // the slot lists of every replica, the fix-up beside the tiles (see
+    // enqueue_tick).
+    const StepArgs* targs = b->d_targs + (size_t)s * b->reps.size();
+    if (b->slot_ctas) {
+        cudaEventRecord(b->ev_fix, b->stream);
+        cudaStreamWaitEvent(b->side, b->ev_fix, 0);
+        b->ops.fixup_list_batch(targs, b->d_bmap, (unsigned)b->nb, b->side);
+        cudaEventRecord(b->ev_list, b->side);
+        batch_particles(b, s);
+    }
     if (b->tuning.tile_cta)
-        b->ops.bulk_batch(b->d_targs + (size_t)s * b->reps.size(), b->d_dmap, b->nd, b->stream,
+        b->ops.bulk_batch(targs, b->d_dmap, b->nd, b->stream,
                           b->reps[0]->rounding == LBM_ROUND_STOCHASTIC, s == 1);
     else
         batch_launch(b, s, batch_items(b, false, false, false, true, 0), 0, b->stream);
+    if (b->slot_ctas) {
+        cudaStreamWaitEvent(b->stream, b->ev_list, 0);
+        b->ops.fixup_store_batch(targs, (unsigned)b->reps.size(), b->slot_ctas, b->stream);
+        return;
+    }
     if (b->part_pending) {
         cudaStreamWaitEvent(b->stream, b->ev_part, 0);
         b->part_pending = false;
@@ -2840,9 +3005,7 @@ void batch_enqueue(lbm_batch* b, int s) {
     if (b->nc > 0) {
         cudaEventRecord(b->ev_fix, b->stream);
         cudaStreamWaitEvent(b->side, b->ev_fix, 0);
-        batch_launch(b, s, batch_items(b, false, false, true, false, 0), 1, b->side);
-        cudaEventRecord(b->ev_part, b->side);
-        b->part_pending = true;
+        batch_particles(b, s);
     }
 }
 
@@ -2864,7 +3027,7 @@ int batch_graph(lbm_batch* b, int s0) {
         cudaGetLastError();
         return bset_err(b, LBM_ERR_CUDA, std::string("graph capture failed: ") + cudaGetErrorString(e));
     }
-    e = cudaGraphInstantiate(&b->graphs[s0], graph, 0);
+    e = cudaGraphInstantiate(&b->graphs[s0], graph, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
         b->graphs[s0] = nullptr;
@@ -2966,6 +3129,7 @@ void batch_destroy_all(lbm_batch* b) {
     if (b->t_end) cudaEventDestroy(b->t_end);
     if (b->ev_fix) cudaEventDestroy(b->ev_fix);
     if (b->ev_part) cudaEventDestroy(b->ev_part);
+    if (b->ev_list) cudaEventDestroy(b->ev_list);
     if (b->side) cudaStreamDestroy(b->side);
     if (b->stream) cudaStreamDestroy(b->stream);
     for (lbm_handle* h : b->reps) destroy_all(h);
@@ -3028,7 +3192,8 @@ int lbm_batch_create(int32_t n, const lbm_config* cfgs, const int32_t* nparticle
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithPriority(&b->side, cudaStreamNonBlocking, hi) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_fix, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->ev_part, cudaEventDisableTiming) != cudaSuccess)
+        cudaEventCreateWithFlags(&b->ev_part, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->ev_list, cudaEventDisableTiming) != cudaSuccess)
         rc = bset_err(b, LBM_ERR_CUDA, "stream or event creation failed");
     if (!rc) rc = bdev_alloc(b, &b->d_targs, sizeof(StepArgs) * 2 * n);
     if (!rc) rc = bdev_alloc(b, &b->d_pargs, sizeof(ParticleArgs) * 2 * n);

@@ -18,6 +18,11 @@ struct Ops {
     // start while the kernel before it in the stream still runs)
     // walk: the chunk-walking kernel (k_fixup_walk), whose grid is fixup_walk_grid
     void (*fixup)(const StepArgs&, unsigned grid, cudaStream_t, bool early, bool walk);
+    // beside the bulk pass: the link slots' values to the list, and their stores after it
+    void (*fixup_list)(const StepArgs&, unsigned grid, cudaStream_t);
+    void (*fixup_store)(const StepArgs&, cudaStream_t, bool early);
+    void (*fixup_list_batch)(const StepArgs* args, const int2* bmap, unsigned blocks, cudaStream_t);
+    void (*fixup_store_batch)(const StepArgs* args, unsigned replicas, unsigned ctas, cudaStream_t);
     void (*particles)(const ParticleArgs&, unsigned grid, cudaStream_t);
     // link-list rebuild of flagged particles: two passes of blocks_per_particle
     // CTAs per particle; counts holds nparts * blocks_per_particle ints
@@ -67,18 +72,34 @@ struct OpsImpl {
     static void bulk(const StepArgs& a, unsigned grid, dim3 block, cudaStream_t s) {
         k_bulk<L, ST, TRT><<<grid, block, 0, s>>>(a);
     }
-    static void fixup(const StepArgs& a, unsigned grid, cudaStream_t s, bool early, bool walk) {
+    template <class K>
+    static void launch_early(K kernel, const StepArgs& a, unsigned grid, int block, cudaStream_t s, bool early) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(kFixThreads);
+        cfg.blockDim = dim3((unsigned)block);
         cfg.stream = s;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = early ? 1 : 0;
-        if (walk) cudaLaunchKernelEx(&cfg, k_fixup_walk<L, ST, TRT>, a);
-        else cudaLaunchKernelEx(&cfg, k_fixup<L, ST, TRT>, a);
+        cudaLaunchKernelEx(&cfg, kernel, a);
+    }
+    static void fixup(const StepArgs& a, unsigned grid, cudaStream_t s, bool early, bool walk) {
+        if (walk) launch_early(k_fixup_walk<L, ST, TRT>, a, grid, kFixThreads, s, early);
+        else launch_early(k_fixup<L, ST, TRT>, a, grid, kFixThreads, s, early);
+    }
+    static void fixup_list(const StepArgs& a, unsigned grid, cudaStream_t s) {
+        k_fixup_walk<L, ST, TRT, true><<<grid, kListThreads, 0, s>>>(a);
+    }
+    static void fixup_store(const StepArgs& a, cudaStream_t s, bool early) {
+        launch_early(k_fixup_store<L, ST>, a, fixup_store_ctas(a.slot_cap), kStoreThreads, s, early);
+    }
+    static void fixup_list_batch(const StepArgs* args, const int2* bmap, unsigned blocks, cudaStream_t s) {
+        k_fixup_batch<L, ST, TRT, kTickBlock><<<blocks, kTickBlock, 0, s>>>(args, bmap);
+    }
+    static void fixup_store_batch(const StepArgs* args, unsigned replicas, unsigned ctas, cudaStream_t s) {
+        k_fixup_store_batch<L, ST><<<dim3(ctas, replicas), kStoreThreads, 0, s>>>(args);
     }
     static void particles(const ParticleArgs& a, unsigned grid, cudaStream_t s) {
         k_particles<L><<<grid, kPartBlock, 0, s>>>(a);
@@ -193,6 +214,10 @@ struct OpsImpl {
         Ops o;
         o.bulk = bulk;
         o.fixup = fixup;
+        o.fixup_list = fixup_list;
+        o.fixup_store = fixup_store;
+        o.fixup_list_batch = fixup_list_batch;
+        o.fixup_store_batch = fixup_store_batch;
         o.particles = particles;
         o.links = links;
         o.encode = encode;
