@@ -99,7 +99,7 @@ __device__ __forceinline__ bool fixup_body(const StepArgs& a, const long long b)
     __shared__ R s_g[Q][kFixBlock];      // post-collision populations of the entries (f/w - rho0)
     __shared__ double s_rho[kFixBlock];  // rho^n of the entries
     __shared__ int s_cell[kFixBlock];
-    __shared__ int s_xyz[3][kFixBlock];
+    __shared__ int s_xyz[3][kFixBlock];  // x with kOnWall and kNoneNear
     __shared__ double s_C[3][3][kFixBlock];  // coordinate of x-1, x, x+1 per axis
     __shared__ unsigned short s_list[kFixBlock * Q];  // (entry << 5) | j of every link slot
     __shared__ R s_val[LIST ? 1 : kFixBlock * Q];     // the value of each listed slot
@@ -168,6 +168,12 @@ __device__ __forceinline__ bool fixup_body(const StepArgs& a, const long long b)
     NodeState<L, ST, TRT> st;
     double cc[3][3];
     int xyz[3] = {0, 0, 0};
+    // kOnWall: the node is a wall node; kNoneNear (wall links): no particle near its tile.
+    // Read here, in one go with the populations, they spare every link slot two
+    // loads in a row (D3Q27 channel of 90 x 62 x 46 nodes with two particles,
+    // 8.3 k wall links: fix-up 12.3 -> 8.2 us, tick 21.6 -> 18.6)
+    constexpr int kOnWall = 1 << 30, kNoneNear = 1 << 29;  // above any x index
+    int flags = 0;
     if (valid) {
         const int cell = ent.x;
         xyz[0] = cell % nx;
@@ -179,6 +185,14 @@ __device__ __forceinline__ bool fixup_body(const StepArgs& a, const long long b)
 #pragma unroll
             for (int o = 0; o < 3; ++o)
                 cc[k][o] = k < D ? a.coord[k][wrap_idx(xyz[k] + o - 1, a.g.n[k])] : 0.0;
+        if (a.wall && a.wall[cell]) flags = kOnWall;
+        if (!is_part) {
+            unsigned long long near = 0;
+            const int tile = xyz[0] / a.g.t[0] + a.g.nt[0] * (xyz[1] / a.g.t[1] + a.g.nt[1] * (xyz[2] / a.g.t[2]));
+            if (a.nparts > 0)
+                for (int w = 0; w < a.words; ++w) near |= a.tilebits[(long long)tile * a.words + w];
+            if (near == 0) flags |= kNoneNear;
+        }
     }
     // break rule of the Ladd loop (fluids.jl:184): for streaming direction j
     // only particles before the first one without links in j contribute.
@@ -189,7 +203,7 @@ __device__ __forceinline__ bool fixup_body(const StepArgs& a, const long long b)
         const unsigned none = ~Pq.dirlinks;
         for (int j = 0; j < Q; ++j)
             if ((none >> j) & 1u) atomicMin(&s_first[j], q);
-        if (is_part && q != p && !a.wall) {
+        if (is_part && q != p) {
             bool meet = true;
             for (int k = 0; k < D; ++k) {
                 // near boxes [slo-1, shi+1] on a periodic axis of n nodes
@@ -205,7 +219,6 @@ __device__ __forceinline__ bool fixup_body(const StepArgs& a, const long long b)
             if (meet) s_alone = 0;
         }
     }
-    if (is_part && a.wall && tid == 0) s_alone = 0;
     // collide each entry's node once
     if (valid) {
         st.rho = collide_node<L, ST, TRT>(a, ent.x, true, st.g);
@@ -215,7 +228,7 @@ __device__ __forceinline__ bool fixup_body(const StepArgs& a, const long long b)
         for (int i = 0; i < Q; ++i) s_g[i][tid] = st.g[i] * R(a.inv_scale);  // storage -> f/w - rho0
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            s_xyz[k][tid] = xyz[k];
+            s_xyz[k][tid] = k == 0 ? xyz[k] | flags : xyz[k];
 #pragma unroll
             for (int o = 0; o < 3; ++o) s_C[k][o][tid] = cc[k][o];
         }
@@ -254,10 +267,10 @@ __device__ __forceinline__ bool fixup_body(const StepArgs& a, const long long b)
             const int i = s_lat[3][j];  // x - c_j = x + c_i is the solid source node
             const int ci0 = s_lat[0][i], ci1 = s_lat[1][i], ci2 = s_lat[2][i];
             R vout;
-            if (a.wall && a.wall[cell]) {
+            if (s_xyz[0][el] & kOnWall) {
                 vout = R(-a.rho0);  // wall nodes hold f = 0 (fluids.jl:154)
             } else {
-                const int x = s_xyz[0][el], y = s_xyz[1][el], z = s_xyz[2][el];
+                const int x = s_xyz[0][el] & (kNoneNear - 1), y = s_xyz[1][el], z = s_xyz[2][el];
                 const double rhoL = s_rho[el];
                 const double gi = (double)s_g[i][el];
                 const double wi = s_w[i];
@@ -273,7 +286,7 @@ __device__ __forceinline__ bool fixup_body(const StepArgs& a, const long long b)
                 // Ladd terms (fluids.jl:176-189) of every particle with link (x, j), in order
                 if (alone) {
                     if (p < s_first[j]) ladd_link<D>(a, sP, true, ci0, ci1, ci2, Tc, Xc, rhoL, gi, wi, v, acc);
-                } else {
+                } else if (!(s_xyz[0][el] & kNoneNear)) {
                     const int tile = x / a.g.t[0] + a.g.nt[0] * (y / a.g.t[1] + a.g.nt[1] * (z / a.g.t[2]));
                     int w = 0;
                     unsigned long long bits = 0;
