@@ -134,8 +134,11 @@ typedef struct lbm_config {
 
 /* Kernel schedule of a tick.  Results do not depend on it (the per-node
  * arithmetic is the same).
+ *   AUTO        (default) small 2D models with FP32 or FP64 storage: many
+ *               ticks in one launch; every other model: STREAM
  *   STREAM      bulk -> fix-up in stream order, particle update on a side
- *               stream overlapping the next bulk pass (AUTO: the default)
+ *               stream overlapping the next bulk pass; with many particles
+ *               the fix-up too, except for its stores
  *   PERSISTENT  one persistent kernel per tick over a work queue of bulk
  *               tiles, fix-up blocks and particle updates (vector bulk kernel
  *               with rows of at most 256 nodes; otherwise STREAM)
@@ -362,7 +365,8 @@ typedef struct lbm_profile {
 } lbm_profile;
 
 /* level 0: off; 1: device time of each lbm_step call; 2: also per-kernel
- * durations (event nodes around every kernel of the step graph) */
+ * durations (event nodes around every kernel of the step graph, which then
+ * runs them one behind the other as in STREAM with few particles) */
 int lbm_set_profiling(lbm_handle* h, int32_t level);
 int lbm_get_profile(lbm_handle* h, lbm_profile* out);
 
@@ -387,7 +391,7 @@ int lbm_time_kernel(lbm_handle* h, int32_t kernel, int32_t launches, double* avg
  *     is not finite or below -1e-3 (wall nodes hold zero density, as in the
  *     reference, so zero itself cannot be told apart from a failure).
  *   - Every wait inside the persistent tick kernel (LBM_SCHEDULE_PERSISTENT)
- *     gives up after a bounded number of polls and raises LBM_ERR_TIMEOUT.
+ *     and inside the many-tick launches of small 2D models gives up after a bounded number of polls and raises LBM_ERR_TIMEOUT.
  * After either error the model's state is undefined: restore a checkpoint
  * (lbm_load_state) or destroy the handle; the error word is cleared once
  * reported, so the handle itself stays usable.
@@ -412,7 +416,8 @@ int lbm_load_state(lbm_handle* h, const char* path);
  * its own grid, parameters and particles, advanced together: every tick runs
  * all replicas' bulk tiles, boundary fix-up blocks and particle updates as the
  * items of one work queue (tick.cuh), either as one persistent launch per
- * tick or as three queue launches in stream order.  The step loop is replayed
+ * tick or in stream order, with the fix-up and the particle updates beside
+ * the bulk tiles.  The step loop is replayed
  * from CUDA graphs.  No counterpart in the reference, which steps one model
  * per call (parameter sweeps there are loops over modelInit/LBMpropagate!).
  * Every replica must take the vector bulk path: n[0] a multiple of 4, x-rows

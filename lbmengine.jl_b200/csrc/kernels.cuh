@@ -18,9 +18,10 @@
 //      Rodrigues rotation, re-voxelisation and link-list rebuild
 //      (moveParticles!, src/gpu/particles.jl:7-92).
 // Nodes inside a particle stream like fluid, as in the reference (its
-// particle interiors are not reset).  The three run either as separate
-// kernels in stream order or as the items of one persistent kernel per tick
-// (k_tick, tick.cuh), which overlaps the boundary work with the bulk pass.
+// particle interiors are not reset).  The three run as separate kernels
+// (the boundary work behind or beside the bulk pass, fixup.cuh), as phases of
+// one launch of many ticks (k_resident, resident.cuh), or as the items of one
+// persistent kernel per tick (k_tick, tick.cuh).
 #pragma once
 #include <cstdint>
 #include "lattice.cuh"

@@ -2,10 +2,11 @@
 //
 // Host side of the drop-in boundary: validates the resolved modelInit /
 // addSquirmer! keyword sets, owns all device memory of a model, and runs
-// LBMpropagate! as CUDA-graph replays of the tick
-//     k_tick (one persistent kernel: bulk, fix-up and particle update items)
-// or, where it does not apply, k_bulk(_v4) -> k_fixup on the main stream with
-// k_particles on a side stream (see enqueue_tick).
+// LBMpropagate! as launches of many ticks (k_resident: small 2D models) or
+// CUDA-graph replays of the tick:
+//     k_bulk(_v4) -> k_fixup on the main stream with k_particles on a side
+//     stream, or with many particles the fix-up there too (see enqueue_tick),
+// or on request k_tick (one persistent kernel: bulk, fix-up and particle items).
 #include "lbm_b200.h"
 #include "ops.cuh"
 #include "interactions.cuh"
