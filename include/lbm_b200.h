@@ -391,7 +391,8 @@ int lbm_time_kernel(lbm_handle* h, int32_t kernel, int32_t launches, double* avg
  *     is not finite or below -1e-3 (wall nodes hold zero density, as in the
  *     reference, so zero itself cannot be told apart from a failure).
  *   - Every wait inside the persistent tick kernel (LBM_SCHEDULE_PERSISTENT)
- *     and inside the many-tick launches of small 2D models gives up after a bounded number of polls and raises LBM_ERR_TIMEOUT.
+ *     and at the grid-wide barrier of small 2D models' launches gives up after
+ *     a bounded number of polls and raises LBM_ERR_TIMEOUT.
  * After either error the model's state is undefined: restore a checkpoint
  * (lbm_load_state) or destroy the handle; the error word is cleared once
  * reported, so the handle itself stays usable.

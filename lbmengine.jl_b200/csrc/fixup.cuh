@@ -392,11 +392,13 @@ __global__ void __launch_bounds__(LIST ? kListThreads : kFixThreads, 512 / (LIST
 // follow the bulk pass is the store of the listed values, a few microseconds
 // (k_fixup_store).  Only the chain store -> next bulk pass stays on the main
 // stream.  64 particles of r = 6 in 192^3 (BF16):
-// 132 -> 107 us per tick; 128 D2Q9 replicas of 64^2 to 256^2 62 -> 47.6.
+// 132 -> 107-112 us per tick; 128 D2Q9 replicas of 64^2 to 256^2 62 -> 47.6.
 // ---------------------------------------------------------------------------
 constexpr int kStoreThreads = 256;
 
-// CTAs that store the list, of `cap` slots at most
+// CTAs that store the list, of `cap` slots at most: two slots per thread, at
+// most four CTAs per SM.  Bound by the scattered stores of single values (260 k
+// of 2 bytes: 4.5-5 us); the loads of the first slot come before the wait.
 __host__ __device__ __forceinline__ unsigned fixup_store_ctas(int cap) {
     const int c = (cap + 2 * kStoreThreads - 1) / (2 * kStoreThreads);
     return (unsigned)(c < 1 ? 1 : (c > 592 ? 592 : c));
