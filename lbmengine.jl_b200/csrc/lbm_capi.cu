@@ -7,6 +7,7 @@
 //     k_bulk(_v4) -> k_fixup on the main stream with k_particles on a side
 //     stream, or with many particles the fix-up there too (see enqueue_tick),
 // or on request k_tick (one persistent kernel: bulk, fix-up and particle items).
+#include <cuda.h>
 #include "lbm_b200.h"
 #include "ops.cuh"
 #include "interactions.cuh"
@@ -409,26 +410,45 @@ cudaError_t read_small(void* dst, const void* src, size_t bytes, cudaStream_t s)
     return e;
 }
 
+// cuPointerGetAttributes through the runtime, which has loaded the driver (null: not found)
+using PointerAttributes = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+PointerAttributes pointer_attributes() {
+    static const PointerAttributes fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &p, 12000, cudaEnableDefault, &found) !=
+                cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<PointerAttributes>(p);
+    }();
+    return fn;
+}
+
 // The device's address of the caller's array where a kernel can write it in
 // place: pinned host memory (cudaHostAlloc, cudaHostRegister) mapped for the
-// current device, from its first to its last byte; else null.
+// current device, all of it in one allocation or registration; else null.  (The
+// ends alone do not tell: an array may span two registrations and a gap that
+// the device cannot reach, and host and device addresses are the same numbers.)
 double* mapped_host(double* host, size_t bytes) {
     if (!host || !bytes) return nullptr;
-    void* dev[2] = {nullptr, nullptr};
-    const char* at[2] = {reinterpret_cast<char*>(host), reinterpret_cast<char*>(host) + bytes - 1};
-    for (int k = 0; k < 2; ++k) {
-        cudaPointerAttributes a{};
-        if (cudaPointerGetAttributes(&a, at[k]) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
-        dev[k] = a.devicePointer;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
     }
-    return static_cast<char*>(dev[1]) - static_cast<char*>(dev[0]) == (long long)bytes - 1 &&
-                   reinterpret_cast<size_t>(dev[0]) % sizeof(double) == 0
-               ? static_cast<double*>(dev[0])
-               : nullptr;
+    if (a.type != cudaMemoryTypeHost || !a.devicePointer || reinterpret_cast<size_t>(a.devicePointer) % sizeof(double))
+        return nullptr;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute which[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* range[2] = {&start, &size};
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(a.devicePointer);
+    if (!pointer_attributes() || pointer_attributes()(2, which, range, at) != CUDA_SUCCESS) return nullptr;
+    return at >= start && at - start <= size && bytes <= size - (at - start) ? static_cast<double*>(a.devicePointer)
+                                                                              : nullptr;
 }
 
 bool get_ops(int lattice, int storage, int trt, Ops* o) {
