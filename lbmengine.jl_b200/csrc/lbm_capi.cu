@@ -375,7 +375,8 @@ struct PinnedChunks {
 PinnedChunks g_pinned;
 struct PinnedLease {
     void* p = nullptr;
-    explicit PinnedLease(size_t bytes) {
+    // allocate false: only a chunk that is there already
+    PinnedLease(size_t bytes, bool allocate) {
         if (bytes > kPinnedChunk) return;  // the caller copies to pageable memory
         {
             std::lock_guard<std::mutex> lk(g_pinned.mu);
@@ -385,7 +386,7 @@ struct PinnedLease {
                 return;
             }
         }
-        if (cudaHostAlloc(&p, kPinnedChunk, cudaHostAllocPortable) != cudaSuccess) {
+        if (allocate && cudaHostAlloc(&p, kPinnedChunk, cudaHostAllocPortable) != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
         }
@@ -400,9 +401,9 @@ struct PinnedLease {
 };
 
 // copy `bytes` from the device through a pinned chunk into `dst`, after the
-// stream's queued work
-cudaError_t read_small(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-    PinnedLease l(bytes);
+// stream's queued work; where none is free and `allocate` is false, straight into `dst`
+cudaError_t read_small(void* dst, const void* src, size_t bytes, cudaStream_t s, bool allocate = true) {
+    PinnedLease l(bytes, allocate);
     cudaError_t e = cudaMemcpyAsync(l.p ? l.p : dst, src, bytes, cudaMemcpyDeviceToHost, s);
     const cudaError_t e2 = cudaStreamSynchronize(s);  // also after an error: the chunk goes back to the pool
     if (e == cudaSuccess) e = e2;
@@ -1310,10 +1311,11 @@ int ensure_graphs(lbm_handle* h, int64_t nsteps) {
 
 // Read (and clear) the device error word after the work of a call.  The state
 // of the model after any of these errors is undefined: restore a checkpoint
-// (lbm_load_state) or destroy the handle.
-int check_device_error(lbm_handle* h) {
+// (lbm_load_state) or destroy the handle.  allocate false: without allocating
+// pinned memory (lbm_step_noalloc).
+int check_device_error(lbm_handle* h, bool allocate = true) {
     int err = 0;
-    CUDA_TRY(h, read_small(&err, h->d_err, sizeof(int), h->stream));
+    CUDA_TRY(h, read_small(&err, h->d_err, sizeof(int), h->stream, allocate));
     if (err == 0) return LBM_OK;
     h->res_ready = false;  // a launch that gave up may have left its masks set
     CUDA_TRY(h, cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
@@ -2793,7 +2795,7 @@ int lbm_step_noalloc(lbm_handle* h, int64_t nsteps) {
     CUDA_TRY(h, cudaGetLastError());
     for (int64_t s = 0; s < nsteps; ++s) h->time += h->dt;
     h->tick += nsteps;
-    return check_device_error(h);
+    return check_device_error(h, false);
 }
 
 void lbm_destroy(lbm_handle* h) { destroy_all(h); }
