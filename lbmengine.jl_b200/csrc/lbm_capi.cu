@@ -117,6 +117,8 @@ struct lbm_handle {
     void* d_slot_val = nullptr;
     int* d_slot_n = nullptr;
     int slot_cap = 0;
+    long long slot_alloc = 0;           // slots the two arrays hold
+    bool slot_refused = false;          // no memory for the present particles' list
     // many ticks per launch (resident.cuh)
     bool auto_schedule = false;         // the caller left the schedule to the library
     int res_ctas = -1;                  // CTAs of the launch; 0: does not apply, -1: not looked up yet
@@ -822,18 +824,31 @@ long long slot_bound(const lbm_handle* h) {
     return n;
 }
 
-// The list of link slots, sized for the model's particles; without the memory
-// (or past 2^30 slots) the fix-up stays behind the bulk pass (slot_cap 0).
-int slot_list(lbm_handle* h) {
-    const long long n = slot_bound(h);
-    if (n <= h->slot_cap || n >= (1LL << 30)) return LBM_OK;
+void free_slot_list(lbm_handle* h) {
+    if (h->d_slot_at) h->device_bytes -= sizeof(long long) * (size_t)h->slot_alloc;
+    if (h->d_slot_val) h->device_bytes -= (size_t)storage_bytes(h->storage) * h->slot_alloc;
+    if (h->d_slot_n) h->device_bytes -= 2 * sizeof(int);
     dev_free(h->d_slot_at);
     dev_free(h->d_slot_val);
+    dev_free(h->d_slot_n);
     h->slot_cap = 0;
-    if (block_alloc((void**)&h->d_slot_at, sizeof(long long) * n) != cudaSuccess ||
-        block_alloc((void**)&h->d_slot_val, (size_t)storage_bytes(h->storage) * n) != cudaSuccess ||
-        (!h->d_slot_n && block_alloc((void**)&h->d_slot_n, 2 * sizeof(int)) != cudaSuccess)) {
-        cudaGetLastError();
+}
+
+// The list of link slots, sized for the model's particles; without the memory
+// (or past 2^30 slots) the fix-up stays behind the bulk pass (slot_cap 0),
+// which is not tried again until a particle is added.
+int slot_list(lbm_handle* h) {
+    const long long n = slot_bound(h);
+    if (n <= h->slot_cap || n >= (1LL << 30) || h->slot_refused) return LBM_OK;
+    h->slot_alloc = n;
+    const std::string err = h->err;
+    int rc = dev_alloc(h, &h->d_slot_at, sizeof(long long) * (size_t)n);
+    if (!rc) rc = dev_alloc(h, (char**)&h->d_slot_val, (size_t)storage_bytes(h->storage) * n);
+    if (!rc) rc = dev_alloc(h, &h->d_slot_n, 2 * sizeof(int));
+    if (rc) {
+        free_slot_list(h);
+        h->slot_refused = true;
+        h->err = err;
         return LBM_OK;
     }
     CUDA_TRY(h, cudaMemsetAsync(h->d_slot_n, 0, 2 * sizeof(int), h->stream));
@@ -2006,6 +2021,8 @@ int lbm_add_particle(lbm_handle* h, const lbm_particle_params* p, int32_t* id_ou
     if (rc) return rc;
     CUDA_TRY(h, cudaMemcpyAsync(h->d_parts + pid, &P, sizeof(P), cudaMemcpyHostToDevice, h->stream));
     h->hparts.push_back(P);
+    free_slot_list(h);  // it was sized for the particles before
+    h->slot_refused = false;
     h->maxchunks = std::max<int>(h->maxchunks, (int)chunks);
     h->link_bpp = std::max<int>(h->link_bpp, (int)((near + kLinkBlock - 1) / kLinkBlock));
     rc = grow(h, &h->d_linkcnt, &h->linkcnt_slots, (long long)(pid + 1) * h->link_bpp, 0);
