@@ -3715,15 +3715,21 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
     AdjState* st = nullptr;
     // the stored states in one block where it fits (a run holds up to min(snapshots, ticks + 1) of them)
     char* arena = nullptr;
+    size_t held = 0;  // device bytes of this call's buffers
+    auto take = [&](auto** p, size_t bytes) {
+        const int r = dev_alloc(h, p, bytes);
+        if (!r) held += bytes;
+        return r;
+    };
     const size_t slots = (size_t)std::min<long long>(spec->snapshots, T + 1);
-    if (dev_alloc(h, &arena, R.snap_bytes * slots) == LBM_OK)
+    if (take(&arena, R.snap_bytes * slots) == LBM_OK)
         for (size_t k = slots; k-- > 0;) R.spare.push_back(arena + k * R.snap_bytes);
-    int rc = dev_alloc(h, &R.lam[0], lam_bytes);
-    if (!rc) rc = dev_alloc(h, &R.lam[1], lam_bytes);
-    if (!rc) rc = dev_alloc(h, &dmu, sizeof(double) * h->N);
-    if (!rc) rc = dev_alloc(h, &partial, part_bytes);
-    if (!rc) rc = dev_alloc(h, &st, sizeof(AdjState));
-    if (!rc) rc = dev_alloc(h, &h->d_rec, rec_bytes);
+    int rc = take(&R.lam[0], lam_bytes);
+    if (!rc) rc = take(&R.lam[1], lam_bytes);
+    if (!rc) rc = take(&dmu, sizeof(double) * h->N);
+    if (!rc) rc = take(&partial, part_bytes);
+    if (!rc) rc = take(&st, sizeof(AdjState));
+    if (!rc) rc = take(&h->d_rec, rec_bytes);
     if (!rc && (cudaMemsetAsync(R.lam[0], 0, lam_bytes, h->stream) != cudaSuccess ||
                 cudaMemsetAsync(dmu, 0, sizeof(double) * h->N, h->stream) != cudaSuccess ||
                 cudaMemsetAsync(st, 0, sizeof(AdjState), h->stream) != cudaSuccess ||
@@ -3789,7 +3795,6 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
         }
     }
     cudaStreamSynchronize(h->stream);  // nothing below is in use any more, after an error either
-    h->device_bytes -= R.snap_bytes * (R.extra.size() + (arena ? slots : 0));
     dev_free(arena);
     for (char*& s : R.extra) dev_free(s);
     if (cudaMemcpy(&h->d_parts[0].recordF, &record_before, sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess &&
@@ -3802,8 +3807,7 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
     dev_free(st);
     dev_free(h->d_rec);
     drop_graphs(h);  // they write the history
-    h->device_bytes -= 2 * lam_bytes + sizeof(double) * h->N + part_bytes + sizeof(AdjState) +
-                       rec_bytes;
+    h->device_bytes -= held + R.snap_bytes * R.extra.size();
     if (rc) return rc;
     std::memset(out, 0, sizeof(*out));
     const double K = (double)(spec->window_end - spec->window_begin + 1);

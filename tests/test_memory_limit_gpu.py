@@ -55,3 +55,26 @@ def test_slot_lists_keep_to_the_limit(lib):
             assert held.info().device_bytes == before
     free.step(5)
     np.testing.assert_array_equal(held.distributions, free.distributions)
+
+
+def _swimmer(**kw):
+    import lbmengine as lbm
+    m = lbm.modelInit(dims=3, latticeParameter=1.0, relaxationTimeRatio=0.8, collisionModel="trt",
+                      xlims=(-10.0, 9.0), ylims=(-10.0, 9.0), zlims=(-10.0, 9.0), **kw)
+    lbm.addSquirmer(m, radius=4.0, position=[0.3, 0.1, -0.2], massDensity=2.0, swimmingSpeed=1e-3, beta=2.0,
+                    coupleForces=True, coupleTorques=True)
+    return m
+
+
+@pytest.mark.parametrize("extra", [1000, 3_000_000])  # no room for the stored states; for some of the buffers
+def test_refused_gradient_gives_its_bytes_back(lib, extra):
+    from lbmengine.adjoint import swimming_speed_gradient
+    m = _swimmer()
+    before = m.info().device_bytes
+    with limit(lib, before + extra), pytest.raises(capi.LbmError) as e:
+        swimming_speed_gradient(m, 6, (4, 6), snapshots=3)
+    assert e.value.code == capi.LBM_ERR_OOM
+    assert m.info().device_bytes == before
+    out = swimming_speed_gradient(m, 6, (4, 6), snapshots=3)
+    assert m.info().device_bytes == before
+    assert out.value == swimming_speed_gradient(_swimmer(), 6, (4, 6), snapshots=3).value
