@@ -128,7 +128,6 @@ struct lbm_handle {
     unsigned *d_pmask = nullptr, *d_wmask = nullptr;
     int* d_rsync = nullptr;             // barrier counter and last phase, then the particles' boxes
     double* d_rpos = nullptr;           // [2][particles][3]
-    int res_parts = 0;                  // particles the two hold
     void* pop[2] = {nullptr, nullptr};
     int cur = 0;
     double* d_coord[3] = {nullptr, nullptr, nullptr};
@@ -964,6 +963,8 @@ constexpr long long kResidentNodesPart = 1ll << 19;
 constexpr long long kResidentNodesWalls = 1ll << 18;
 constexpr long long kResidentNodesFluid = (kResMaxCluster - 1) * kResThreads;
 constexpr int64_t kResidentTicks = 4096;  // ticks per launch
+constexpr size_t kResSyncBytes = sizeof(int) * (2 + 6 * kResMaxParts);  // barrier, then the particles' boxes
+constexpr size_t kResPosBytes = sizeof(double) * 6 * kResMaxParts;
 
 // Shared memory of a boundary CTA: bounds that no particle of its radius
 // exceeds (a cluster launch cannot end early).  The link nodes lie less than
@@ -1026,6 +1027,56 @@ int resident_clusters(const lbm_handle* h, size_t smem, int csize) {
     return clusters;
 }
 
+// the job of model h whose first tick reads buffer `src`
+ResidentJob resident_job(const lbm_handle* h, int src) {
+    ResidentJob j{};
+    for (int s = 0; s < 2; ++s) j.a[s] = step_args(h, src ^ s);
+    j.pa = particle_args(h, 0, 0);  // publishes the box into both buffers
+    j.pa.inline_links = 1;
+    j.in = inter_args(h);
+    j.pmask = h->d_pmask;
+    j.wmask = h->has_walls ? h->d_wmask : nullptr;
+    j.box = h->d_rsync + 2;
+    j.pos = h->d_rpos;
+    return j;
+}
+
+void free_resident(lbm_handle* h) {
+    if (h->d_pmask) h->device_bytes -= 2 * sizeof(unsigned) * h->N;
+    if (h->d_wmask) h->device_bytes -= sizeof(unsigned) * h->N;
+    if (h->d_rjobs) h->device_bytes -= 2 * sizeof(ResidentJob);
+    if (h->d_rsync) h->device_bytes -= kResSyncBytes;
+    if (h->d_rpos) h->device_bytes -= kResPosBytes;
+    dev_free(h->d_pmask);
+    dev_free(h->d_wmask);
+    dev_free(h->d_rjobs);
+    dev_free(h->d_rsync);
+    dev_free(h->d_rpos);
+}
+
+// the device buffers of resident launches: masks of the pushes they leave out, jobs, barrier, particle boxes
+int resident_buffers(lbm_handle* h) {
+    int rc = LBM_OK;
+    const bool new_wmask = h->has_walls && !h->d_wmask;
+    if (!h->d_pmask) rc = dev_alloc(h, &h->d_pmask, 2 * sizeof(unsigned) * h->N);
+    if (!rc && !h->d_rjobs) rc = dev_alloc(h, &h->d_rjobs, 2 * sizeof(ResidentJob));
+    if (!rc && !h->d_rsync) rc = dev_alloc(h, &h->d_rsync, kResSyncBytes);
+    if (!rc && !h->d_rpos) rc = dev_alloc(h, &h->d_rpos, kResPosBytes);
+    if (!rc && new_wmask) rc = dev_alloc(h, &h->d_wmask, sizeof(unsigned) * h->N);
+    if (rc) return rc;
+    CUDA_TRY(h, cudaMemsetAsync(h->d_pmask, 0, 2 * sizeof(unsigned) * h->N, h->stream));
+    if (new_wmask) {
+        h->ops.resident_wmask(h->d_wall, h->g, h->d_wmask, h->stream);
+        CUDA_TRY(h, cudaGetLastError());
+    }
+    const ResidentJob j[2] = {resident_job(h, 0), resident_job(h, 1)};
+    CUDA_TRY(h, cudaMemcpyAsync(h->d_rjobs, j, sizeof(j), cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    h->res_ready = true;
+    return LBM_OK;
+}
+
+// whether lbm_step runs resident; then the buffers are there and the jobs current
 bool use_resident(lbm_handle* h) {
     if (!h->auto_schedule || h->bulk_kind != LBM_BULK_AUTO || h->profiling >= 2 || !resident_applies(h) ||
         h->N > (!h->hparts.empty() ? kResidentNodesPart : (h->has_walls ? kResidentNodesWalls : kResidentNodesFluid)))
@@ -1051,59 +1102,23 @@ bool use_resident(lbm_handle* h) {
             cudaGetLastError();
         }
     }
-    return h->res_ctas > (int)h->hparts.size();
-}
-
-// the job of model h whose first tick reads buffer `src`
-ResidentJob resident_job(const lbm_handle* h, int src) {
-    ResidentJob j{};
-    for (int s = 0; s < 2; ++s) j.a[s] = step_args(h, src ^ s);
-    j.pa = particle_args(h, 0, 0);  // publishes the box into both buffers
-    j.pa.inline_links = 1;
-    j.in = inter_args(h);
-    j.pmask = h->d_pmask;
-    j.wmask = h->has_walls ? h->d_wmask : nullptr;
-    j.box = h->d_rsync + 2;
-    j.pos = h->d_rpos;
-    return j;
-}
-
-// the device buffers of resident launches: masks of the pushes they leave out, jobs, barrier, particle boxes
-int resident_buffers(lbm_handle* h) {
-    int rc = LBM_OK;
-    const int np = (int)h->hparts.size();
-    if (!h->d_pmask) rc = dev_alloc(h, &h->d_pmask, 2 * sizeof(unsigned) * h->N);
-    if (!rc && !h->d_rjobs) rc = dev_alloc(h, &h->d_rjobs, 2 * sizeof(ResidentJob));
-    if (!rc && (!h->d_rsync || h->res_parts < np)) {
-        dev_free(h->d_rsync);
-        dev_free(h->d_rpos);
-        rc = dev_alloc(h, &h->d_rsync, sizeof(int) * (2 + 6 * kResMaxParts));
-        if (!rc) rc = dev_alloc(h, &h->d_rpos, sizeof(double) * 6 * kResMaxParts);
-        h->res_parts = kResMaxParts;
+    if (h->res_ctas <= (int)h->hparts.size()) return false;
+    if (!h->res_ready) {
+        const std::string err = h->err;
+        if (resident_buffers(h) != LBM_OK) {  // no memory: the stream schedule, which needs none
+            free_resident(h);
+            h->res_ctas = 0;
+            h->err = err;
+            return false;
+        }
     }
-    if (rc) return rc;
-    CUDA_TRY(h, cudaMemsetAsync(h->d_pmask, 0, 2 * sizeof(unsigned) * h->N, h->stream));
-    if (h->has_walls && !h->d_wmask) {
-        rc = dev_alloc(h, &h->d_wmask, sizeof(unsigned) * h->N);
-        if (rc) return rc;
-        h->ops.resident_wmask(h->d_wall, h->g, h->d_wmask, h->stream);
-        CUDA_TRY(h, cudaGetLastError());
-    }
-    return LBM_OK;
+    return true;
 }
 
 // up to nsteps ticks; *ran: how many (fewer where a launch ended early).  The
 // buffers swap roles after an odd number.
 int resident_ticks(lbm_handle* h, int64_t nsteps, int64_t* ran) {
     *ran = 0;
-    if (!h->res_ready) {
-        const int rc = resident_buffers(h);
-        if (rc) return rc;
-        const ResidentJob j[2] = {resident_job(h, 0), resident_job(h, 1)};
-        CUDA_TRY(h, cudaMemcpyAsync(h->d_rjobs, j, sizeof(j), cudaMemcpyHostToDevice, h->stream));
-        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-        h->res_ready = true;
-    }
     const ResidentCaps caps = resident_caps(h);
     const bool may_stop = h->hparts.size() > 1;  // a launch can end early
     while (*ran < nsteps) {

@@ -78,3 +78,26 @@ def test_refused_gradient_gives_its_bytes_back(lib, extra):
     out = swimming_speed_gradient(m, 6, (4, 6), snapshots=3)
     assert m.info().device_bytes == before
     assert out.value == swimming_speed_gradient(_swimmer(), 6, (4, 6), snapshots=3).value
+
+
+@pytest.mark.parametrize("walls", [False, True])
+@pytest.mark.parametrize("extra", [16, 24_600])  # no room for any buffer of the many-ticks launch; for the masks alone
+def test_small_model_at_the_limit_steps_in_stream_order(lib, walls, extra):
+    import lbmengine as lbm
+
+    def model(schedule):
+        m = lbm.modelInit(dims=2, latticeParameter=1.0, relaxationTimeRatio=0.8, schedule=schedule,
+                          xlims=(-32.0, 31.0), ylims=(-24.0, 23.0), walledDimensions=[2] if walls else [])
+        lbm.addSquirmer(m, radius=6.0, position=[0.3, 0.2], massDensity=3.0, swimmingSpeed=1e-3, beta=2.0,
+                        swimmingDirection=[0.8, 0.6], coupleForces=True, coupleTorques=True)
+        return m
+
+    small, ref = model("auto"), model("stream")
+    before = small.info().device_bytes
+    with limit(lib, before + extra):
+        for n in (3, 40):
+            small.step(n)
+            ref.step(n)
+            assert launches(lib, small) == 3 * n
+    assert small.info().device_bytes == before
+    np.testing.assert_array_equal(small.distributions, ref.distributions)
