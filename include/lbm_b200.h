@@ -397,10 +397,12 @@ int lbm_time_kernel(lbm_handle* h, int32_t kernel, int32_t launches, double* avg
  * (lbm_load_state) or destroy the handle; the error word is cleared once
  * reported, so the handle itself stays usable.
  *
- * lbm_set_wait_limit: `polls` bounds every wait of the tick kernel (1 ..
- * 2^22, the default; a poll sleeps >= 128 ns).  `target_offset` is a test
- * knob: 1 raises the target of the fix-up items' wait above any count the
- * kernel can reach, so that wait runs into the limit; 0 in normal use.
+ * lbm_set_wait_limit: `polls` bounds every wait of the tick kernel and of the
+ * grid-wide barrier (1 .. 2^22, the default; a poll of the tick kernel sleeps
+ * >= 128 ns, one of the barrier reads a counter).  `target_offset` is a test
+ * knob: 1 raises the target of the fix-up items' wait, or of the barrier,
+ * above any count the kernel can reach, so that wait runs into the limit; 0 in
+ * normal use.
  *
  * lbm_set_memory_limit: a process-wide cap on the device bytes any one handle
  * may hold (0, the default: no cap); an allocation beyond it fails with

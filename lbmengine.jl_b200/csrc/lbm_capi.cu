@@ -110,8 +110,8 @@ struct lbm_handle {
     StepArgs* d_targs = nullptr;      // [2]: by source buffer
     ParticleArgs* d_pargs = nullptr;  // [2]
     TickCounters* d_tq = nullptr;
-    long long spin_limit = kSpinLimit;  // polls before a wait of the tick kernel gives up
-    int wait_extra = 0;                 // test knob: added to the fix-up items' wait target
+    long long spin_limit = kSpinLimit;  // polls before a wait of the tick kernel or the grid barrier gives up
+    int wait_extra = 0;                 // test knob: added to the wait target of the fix-up items or the barrier
     // the fix-up beside the bulk pass: the list of link slots (fixup.cuh)
     long long* d_slot_at = nullptr;
     void* d_slot_val = nullptr;
@@ -1130,6 +1130,8 @@ int resident_ticks(lbm_handle* h, int64_t nsteps, int64_t* ran) {
         r.cap_slots = (int)caps.slots;
         r.cap_box = (int)caps.box;
         r.err = h->d_err;
+        r.spin_limit = h->spin_limit;
+        r.wait_extra = (unsigned)h->wait_extra;
         if (h->res_cluster == 0) {
             r.bar = reinterpret_cast<unsigned*>(h->d_rsync);
             CUDA_TRY(h, cudaMemsetAsync(h->d_rsync, 0, sizeof(unsigned), h->stream));
@@ -1352,7 +1354,7 @@ int check_device_error(lbm_handle* h, bool allocate = true) {
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     if (err & kErrLinkOverflow) return set_err(h, LBM_ERR_STATE, "particle boundary links exceeded their capacity");
     if (err & kErrIntervalOverflow) return set_err(h, LBM_ERR_STATE, "particle solid box exceeded its capacity");
-    if (err & kErrSpinTimeout) return set_err(h, LBM_ERR_TIMEOUT, "a wait inside the tick kernel gave up");
+    if (err & kErrSpinTimeout) return set_err(h, LBM_ERR_TIMEOUT, "a bounded wait inside a kernel of the tick gave up");
     if (err & kErrNumeric)
         return set_err(h, LBM_ERR_NUMERIC,
                        "non-finite or negative density on the device (the simulation diverged near tick " +
@@ -3113,7 +3115,7 @@ int batch_check(lbm_batch* b) {
     b->diverged.resize(n, 0);
     for (size_t r = 0; r < n; ++r)
         if (err[r] & kErrNumeric) b->diverged[r] = 1;  // a sweep goes on; lbm_batch_status reports them
-    if (err[n] & kErrSpinTimeout) return bset_err(b, LBM_ERR_TIMEOUT, "a wait inside the tick kernel gave up");
+    if (err[n] & kErrSpinTimeout) return bset_err(b, LBM_ERR_TIMEOUT, "a bounded wait inside a kernel of the tick gave up");
     for (size_t r = 0; r < n; ++r) {
         if (err[r] & kErrLinkOverflow)
             return bset_err(b, LBM_ERR_STATE, "replica " + std::to_string(r) + ": particle links exceeded their capacity");

@@ -48,7 +48,6 @@ constexpr int kResMaxEntries = kResMaxChunks * kFixBlock;    // link entries of 
 constexpr int kResMaxParts = 32;
 constexpr int kResMaxInter = 128;                            // interaction contributions to one particle
 constexpr size_t kResMaxSmem = 200 * 1024;                   // dynamic shared memory per CTA
-constexpr long long kResSpinLimit = 1LL << 22;  // polls of the grid barrier before it gives up (about a second)
 
 struct ResidentJob {
     StepArgs a[2];          // by tick parity
@@ -69,6 +68,8 @@ struct ResidentArgs {
     unsigned* bar;       // grid barrier: counter (zero at launch) and the phase the launch ends at (all
                          // ones at launch); null: cluster barrier
     int* err;            // of the grid barrier
+    long long spin_limit;  // polls before a wait at the grid barrier gives up (2^22: about a second)
+    unsigned wait_extra;   // test knob: added to the count it waits for
 };
 
 __device__ __forceinline__ unsigned cluster_rank() {
@@ -112,6 +113,8 @@ struct ResidentBarrier {
     int* err;
     unsigned phase;     // phases completed
     unsigned ctas;
+    long long limit;    // polls of a wait
+    unsigned extra;
     __device__ __forceinline__ void arrive(bool stop = false) {
         if (ctr) {
             if (threadIdx.x == kResThreads - 32) {
@@ -144,11 +147,11 @@ struct ResidentBarrier {
             long long it = 0;
             while (true) {
                 const unsigned v = load(ctr);
-                if ((v & 0x7fffffffu) >= phase * ctas) {
+                if ((v & 0x7fffffffu) >= phase * ctas + extra) {
                     if ((v & 0x80000000u) && load(ctr + 1) <= phase) state = kStop;
                     break;
                 }
-                if (++it > kResSpinLimit) {
+                if (++it > limit) {
                     atomicOr(err, kErrSpinTimeout);
                     state = kGaveUp;
                     break;
@@ -558,7 +561,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
     __shared__ double s_part[kResMaxChunks][kPartialStride];
     __shared__ double s_red[kResThreads / 32][6];
     __shared__ int s_off[kResMaxChunks + 1];  // first slot of each chunk
-    __shared__ int s_wcnt[2], s_stop, s_box[6];
+    __shared__ int s_wcnt[2], s_stop, s_quit, s_box[6];
     __shared__ int s_nsrc[2];  // source nodes set in each parity's pmask
     __shared__ int s_lat[4][Q];  // c_i (3) and i of the slot direction j, i = opp(j)
     __shared__ double s_w[Q];
@@ -567,7 +570,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
     const bool grid = ra.bar != nullptr;
     const int rank = grid ? (int)blockIdx.x : (int)cluster_rank();
     const int csize = grid ? (int)gridDim.x : (int)cluster_size();
-    ResidentBarrier bar{ra.bar, ra.err, 0u, (unsigned)csize};
+    ResidentBarrier bar{ra.bar, ra.err, 0u, (unsigned)csize, ra.spin_limit, ra.wait_extra};
     for (int j = tid; j < Q; j += kResThreads) {
         s_lat[0][j] = -L::cx(j);
         s_lat[1][j] = -L::cy(j);
@@ -580,8 +583,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
         reinterpret_cast<int*>(s_a)[k] = reinterpret_cast<const int*>(J.a)[k];
     for (int k = tid; k < (int)(sizeof(ParticleArgs) / 4); k += kResThreads)
         reinterpret_cast<int*>(&s_pa)[k] = reinterpret_cast<const int*>(&J.pa)[k];
-    if (tid == 0) s_stop = s_nsrc[0] = s_nsrc[1] = 0;
+    if (tid == 0) {
+        s_stop = s_nsrc[0] = s_nsrc[1] = 0;
+        // a launch before this one of the same call gave up: what it left is undefined
+        s_quit = grid && (*(volatile const int*)ra.err & kErrSpinTimeout) != 0;
+    }
     __syncthreads();
+    if (s_quit) return;
     const int np = s_a[0].nparts;
     const bool walls = s_a[0].nwnodes > 0;
     const int bulk_ctas = csize - np;
