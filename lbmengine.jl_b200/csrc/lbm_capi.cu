@@ -11,6 +11,7 @@
 #include "lbm_b200.h"
 #include "ops.cuh"
 #include "interactions.cuh"
+#include "resident_caps.h"
 
 #include <algorithm>
 #include <cmath>
@@ -966,26 +967,9 @@ constexpr int64_t kResidentTicks = 4096;  // ticks per launch
 constexpr size_t kResSyncBytes = sizeof(int) * (2 + 6 * kResMaxParts);  // barrier, then the particles' boxes
 constexpr size_t kResPosBytes = sizeof(double) * 6 * kResMaxParts;
 
-// Shared memory of a boundary CTA: bounds that no particle of its radius
-// exceeds (a cluster launch cannot end early).  The link nodes lie less than
-// sqrt(2) outside the sphere (their unit squares in a ring), or across the
-// periodic boundary from a sphere clipped at the edges of the box; eight slots
-// each.
-struct ResidentCaps {
-    long long entries = 1, slots = 1, box = 1;
-};
 ResidentCaps resident_caps(const lbm_handle* h) {
     ResidentCaps c;
-    const double pi = 3.14159265358979;
-    for (const ParticleDev& P : h->hparts) {
-        const double r = P.radius / h->dx;
-        const double s2 = std::sqrt(2.0), out = r + 1.5 * s2, in = std::max(0.0, r - 0.5 * s2);
-        const double e = pi * (out * out - in * in) + 4.0 * (2.0 * r + 4.0);
-        c.entries = std::max(c.entries, std::min<long long>(P.link_cap, (long long)std::ceil(e)));
-        c.slots = std::max(c.slots, 8 * (long long)std::ceil(e));
-        for (int k = 0; k < h->dims; ++k)
-            c.box = std::max(c.box, std::min<long long>((long long)std::floor(2.0 * r) + 8, h->n[k]) + 2);
-    }
+    for (const ParticleDev& P : h->hparts) c.add(P.radius / h->dx, h->n, h->dims, P.link_cap);
     return c;
 }
 

@@ -627,6 +627,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
         }
         if (tid == 0) s_nsrc[b] = now;
     };
+    // The links outgrew the shared memory (ResidentCaps says that they cannot).
+    // Several particles: the launch ends after the tick.  One: a cluster cannot
+    // end early, so the call fails instead of going on without the particle.
+    auto outgrown = [&]() {
+        s_stop = 1;
+        if (np == 1) atomicOr(s_a[0].err, kErrLinkOverflow);
+    };
     // Entries, coordinates and slot list of the current links; sets s_stop
     // where this launch cannot go on with them.
     auto relist = [&](bool check_move) {
@@ -661,7 +668,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
         if (tid == 0) {
             s_off[0] = 0;
             resident_keep<D>(s_pa, sP, &s_keep);
-            if (!fits) s_stop = 1;
+            if (!fits) outgrown();
             if (np > 1) {
                 if ((sP.dirlinks & kAllDirs) != kAllDirs) s_stop = 1;
                 for (int k = 0; k < 3; ++k) {
@@ -695,7 +702,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             __syncthreads();
             const int base = s_off[c], end = base + s_wcnt[0] + s_wcnt[1];
             if (end > B.S) {  // the same in every thread
-                if (tid == 0) s_stop = 1;
+                if (tid == 0) outgrown();
                 entries = 0;
                 nch = 0;
                 break;
