@@ -1099,10 +1099,10 @@ bool use_resident(lbm_handle* h) {
     return true;
 }
 
-// up to nsteps ticks; *ran: how many (fewer where a launch ended early).  The
-// buffers swap roles after an odd number.
-int resident_ticks(lbm_handle* h, int64_t nsteps, int64_t* ran) {
-    *ran = 0;
+// up to nsteps ticks; *ran: how many (fewer where a launch ended early),
+// *launched: the launches.  The buffers swap roles after an odd number.
+int resident_ticks(lbm_handle* h, int64_t nsteps, int64_t* ran, int64_t* launched) {
+    *ran = *launched = 0;
     const ResidentCaps caps = resident_caps(h);
     const bool may_stop = h->hparts.size() > 1;  // a launch can end early
     while (*ran < nsteps) {
@@ -1122,6 +1122,7 @@ int resident_ticks(lbm_handle* h, int64_t nsteps, int64_t* ran) {
             CUDA_TRY(h, cudaMemsetAsync(h->d_rsync + 1, 0xff, sizeof(unsigned), h->stream));
         }
         CUDA_TRY(h, h->ops.resident(r, h->res_ctas, h->res_cluster, h->stream));
+        ++*launched;
         int phase = -1;  // the barrier phase the launch ended at (the first one lies before its first tick)
         if (may_stop) CUDA_TRY(h, read_small(&phase, h->d_rsync + 1, sizeof(int), h->stream));
         const bool stopped = phase >= 0;
@@ -2064,8 +2065,9 @@ int lbm_step(lbm_handle* h, int64_t nsteps) {
     if (h->profiling) CUDA_TRY(h, cudaEventRecord(h->t_begin, h->stream));
     int64_t done = 0;
     int slots_used = 0;
+    int64_t launches = 0;
     if (resident) {
-        const int rc = resident_ticks(h, nsteps, &done);
+        const int rc = resident_ticks(h, nsteps, &done, &launches);
         if (rc) return rc;
         if (done < nsteps) {  // a launch ended early: the rest of the call in stream order
             int rc2 = prepare_tick(h);
@@ -2073,6 +2075,7 @@ int lbm_step(lbm_handle* h, int64_t nsteps) {
             if (rc2) return rc2;
         }
     }
+    launches += (nsteps - done) * launches_per_tick(h);
     if (direct) {
         for (; done < nsteps; ++done) {
             enqueue_tick(h, h->cur, (int)done);
@@ -2097,7 +2100,7 @@ int lbm_step(lbm_handle* h, int64_t nsteps) {
     lbm_profile& p = h->prof;
     p = lbm_profile{};
     p.steps = nsteps;
-    p.launches = resident ? (nsteps + kResidentTicks - 1) / kResidentTicks : nsteps * launches_per_tick(h);
+    p.launches = launches;
     p.bulk_cells = h->N;
     if (h->profiling && nsteps > 0) {
         float ms = 0;

@@ -1,0 +1,77 @@
+"""Which schedule a small 2D model's calls take, by the kernel launches that the profile counts: one launch for many
+ticks, more where a launch ends early or a call has more ticks than one launch takes, none of them where the stream
+schedule was asked for."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from lbmengine import _capi as capi
+
+pytestmark = pytest.mark.gpu
+
+MAX_TICKS = 4096  # ticks per launch
+
+
+def _model(n, parts, schedule="auto", walls=False, toward=False, storage="f32"):
+    import lbmengine as lbm
+    nx, ny = n
+    m = lbm.modelInit(dims=2, latticeParameter=1.0, relaxationTimeRatio=0.8, schedule=schedule, storage=storage,
+                      xlims=(-float(nx // 2), float(nx - 1 - nx // 2)), ylims=(-float(ny // 2), float(ny - 1 - ny // 2)),
+                      walledDimensions=[2] if walls else [])
+    for k, pos in enumerate(parts):
+        lbm.addSquirmer(m, radius=6.0, position=pos, massDensity=3.0, swimmingSpeed=8e-3 if toward else 1e-3, beta=2.0,
+                        swimmingDirection=[1.0 - 2.0 * k, 0.0] if toward else [0.8, 0.6], coupleForces=True,
+                        coupleTorques=True)
+    return m
+
+
+def _launches(lib, m, ticks):
+    m.step(ticks)
+    p = capi.LbmProfile()
+    assert lib.lbm_get_profile(m.handle, C.byref(p)) == 0
+    return p.launches
+
+
+ONE = [[0.3, 0.2]]
+APART = [[-20.3, 0.2], [20.1, 0.6]]
+TOUCHING = [[-7.2, 0.0], [7.4, 0.3]]
+
+
+@pytest.mark.parametrize("n,parts,walls", [((48, 40), ONE, False), ((130, 111), ONE, False), ((201, 65), ONE, True),
+                                           ((61, 40), [], True), ((64, 64), [], False), ((120, 90), APART, False)])
+def test_one_launch_per_call(lib, n, parts, walls):
+    m = _model(n, parts, walls=walls)
+    assert [_launches(lib, m, t) for t in (1, 30, MAX_TICKS)] == [1, 1, 1]
+    assert _launches(lib, _model(n, parts, "stream", walls), 30) == 30 * (1 + bool(parts or walls) + bool(parts))
+
+
+@pytest.mark.parametrize("n,parts", [((48, 40), ONE), ((130, 111), ONE), ((120, 90), APART)])
+def test_more_ticks_than_one_launch_takes(lib, n, parts):
+    """From both buffers: after an even and an odd number of ticks.  FP32 populations agree with the stream schedule to
+    a unit in the last place per tick at most, which the flow damps: 1e-6 after some thousand ticks."""
+    for first in (2, 3):
+        a, b = _model(n, parts), _model(n, parts, "stream")
+        for ticks in (first, MAX_TICKS + 5, 2 * MAX_TICKS + 1):
+            assert _launches(lib, a, ticks) == (ticks + MAX_TICKS - 1) // MAX_TICKS
+            b.step(ticks)
+        assert a.tick == b.tick
+        np.testing.assert_allclose(a.distributions, b.distributions, rtol=0, atol=1e-6)
+        for p, q in zip(a.particle_states(), b.particle_states()):
+            np.testing.assert_allclose(list(p.position), list(q.position), rtol=0, atol=1e-6)
+
+
+def test_a_launch_that_ends_early_is_counted_with_what_follows(lib):
+    # boxes of index ranges 30..45 and 51..66; the launch ends where the first one's end + 4 reaches the second one's
+    # start, after 0.2 and 0.4 nodes of approach
+    m, ref = (_model((96, 64), [[-10.2, 0.0], [10.4, 0.3]], s, toward=True) for s in ("auto", "stream"))
+    assert _launches(lib, m, 1) == 1
+    n = _launches(lib, m, 600)  # one launch, then three per tick
+    assert n > 1 and (n - 1) % 3 == 0 and n < 1 + 3 * 600
+    ref.step(1)
+    ref.step(600)
+    np.testing.assert_allclose(m.distributions, ref.distributions, rtol=0, atol=1e-6)
+    touching = _model((96, 64), TOUCHING)
+    assert _launches(lib, touching, 20) == 1 + 3 * 20  # at the first barrier
