@@ -125,6 +125,7 @@ struct lbm_handle {
     int res_ctas = -1;                  // CTAs of the launch; 0: does not apply, -1: not looked up yet
     int res_cluster = 0;                // CTAs per cluster; 0: one cooperative grid
     bool res_ready = false;             // the jobs below are current
+    int64_t res_hold = 0, res_wait = 0; // ticks left in stream order after a launch that ended early, and of the last such wait
     ResidentJob* d_rjobs = nullptr;     // [2]: by the buffer the first tick reads
     unsigned *d_pmask = nullptr, *d_wmask = nullptr;
     int* d_rsync = nullptr;             // barrier counter and last phase, then the particles' boxes
@@ -519,6 +520,7 @@ void drop_graphs(lbm_handle* h) {
     h->tick_ready = false;  // the tick kernel's maps and arguments are rebuilt with the graphs
     h->res_ready = false;
     h->res_ctas = -1;
+    h->res_hold = h->res_wait = 0;
     for (auto& prof : h->graphs)
         for (auto& row : prof)
             for (auto& gr : row) {
@@ -964,6 +966,11 @@ constexpr long long kResidentNodesPart = 1ll << 19;
 constexpr long long kResidentNodesWalls = 1ll << 18;
 constexpr long long kResidentNodesFluid = (kResMaxCluster - 1) * kResThreads;
 constexpr int64_t kResidentTicks = 4096;  // ticks per launch
+// A launch ends early where particles are close, and they stay so for a while:
+// the next kResidentHold ticks run in stream order without another attempt,
+// twice as many each time that one ends before its first tick (an attempt costs
+// two memsets, a cooperative launch and a blocking read).
+constexpr int64_t kResidentHold = 64;
 constexpr size_t kResSyncBytes = sizeof(int) * (2 + 6 * kResMaxParts);  // barrier, then the particles' boxes
 constexpr size_t kResPosBytes = sizeof(double) * 6 * kResMaxParts;
 
@@ -2051,37 +2058,41 @@ int lbm_step(lbm_handle* h, int64_t nsteps) {
     if (!h) return set_err(h, LBM_ERR_INVALID, "null handle");
     if (nsteps < 0) return set_err(h, LBM_ERR_INVALID, "ticks must be non-negative");
     BIND(h);
-    const bool resident = use_resident(h);
-    if (!resident) {
+    const bool resident = h->res_hold <= 0 && use_resident(h);
+    const bool first = h->calls++ == 0;
+    int64_t done = 0, launches = 0;
+    bool direct = false;
+    auto prepare_stream = [&]() {  // for the ticks not done yet
         int rc = prepare_tick(h);
         if (!rc && many_chunks(h) && !use_tick_kernel(h)) rc = slot_list(h);
-        if (rc) return rc;
-    }
-    const bool direct = h->calls++ == 0 && nsteps <= kFirstCallDirectTicks && !resident;
-    if (nsteps > 0 && !direct && !resident) {
-        const int rc = ensure_graphs(h, nsteps);
+        direct = first && nsteps - done <= kFirstCallDirectTicks;
+        if (!rc && done < nsteps && !direct) rc = ensure_graphs(h, nsteps - done);
+        return rc;
+    };
+    if (!resident) {
+        const int rc = prepare_stream();
         if (rc) return rc;
     }
     if (h->profiling) CUDA_TRY(h, cudaEventRecord(h->t_begin, h->stream));
-    int64_t done = 0;
     int slots_used = 0;
-    int64_t launches = 0;
     if (resident) {
-        const int rc = resident_ticks(h, nsteps, &done, &launches);
-        if (rc) return rc;
-        if (done < nsteps) {  // a launch ended early: the rest of the call in stream order
-            int rc2 = prepare_tick(h);
-            if (!rc2) rc2 = ensure_graphs(h, nsteps - done);
-            if (rc2) return rc2;
+        int rc = resident_ticks(h, nsteps, &done, &launches);
+        if (!rc && done < nsteps) {  // a launch ended early: the rest of the call in stream order
+            h->res_wait = done == 0 && h->res_wait > 0 ? std::min(2 * h->res_wait, kResidentTicks) : kResidentHold;
+            h->res_hold = h->res_wait;
+            rc = prepare_stream();
+        } else if (nsteps > 0) {
+            h->res_wait = 0;
         }
+        if (rc) return rc;
     }
+    h->res_hold -= std::min(h->res_hold, nsteps - done);
     launches += (nsteps - done) * launches_per_tick(h);
     if (direct) {
         for (; done < nsteps; ++done) {
-            enqueue_tick(h, h->cur, (int)done);
+            enqueue_tick(h, h->cur, slots_used++);
             h->cur = 1 - h->cur;
         }
-        slots_used = (int)nsteps;
     }
     while (done < nsteps) {
         int k = 0;
@@ -2540,6 +2551,7 @@ int lbm_set_particle(lbm_handle* h, int32_t id, const lbm_particle_state* s) {
         P.w[k] = s->angular_velocity[k];
         P.e[k] = s->swimming_direction[k];
     }
+    h->res_hold = h->res_wait = 0;  // of another place
     CUDA_TRY(h, cudaMemcpyAsync(h->d_parts + (id - 1), &P, sizeof(P), cudaMemcpyHostToDevice, h->stream));
     h->ops.particles(particle_args(h, 1, id - 1), 1, h->stream);
     CUDA_TRY(h, cudaGetLastError());
@@ -2711,6 +2723,7 @@ int lbm_load_state(lbm_handle* h, const char* path) {
          (np == 0 || std::fread(parts.data(), sizeof(ParticleDev), np, fp) == (size_t)np);
     std::fclose(fp);
     if (!ok) return set_err(h, LBM_ERR_INVALID, "truncated checkpoint");
+    h->res_hold = h->res_wait = 0;  // of another state
     // clear the tile bits of the current geometry, then restore and re-voxelise
     CUDA_TRY(h, cudaMemsetAsync(h->d_tilebits, 0, sizeof(unsigned long long) * h->g.ntiles * h->words, h->stream));
     CUDA_TRY(h, cudaMemcpyAsync(h->pop[h->cur], buf.data(), pop_bytes, cudaMemcpyHostToDevice, h->stream));

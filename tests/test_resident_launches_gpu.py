@@ -75,3 +75,19 @@ def test_a_launch_that_ends_early_is_counted_with_what_follows(lib):
     np.testing.assert_allclose(m.distributions, ref.distributions, rtol=0, atol=1e-6)
     touching = _model((96, 64), TOUCHING)
     assert _launches(lib, touching, 20) == 1 + 3 * 20  # at the first barrier
+
+
+def test_close_particles_do_not_pay_for_an_attempt_per_call(lib):
+    """After a launch that ended at its first barrier 64 ticks run in stream order before the next attempt, then 128;
+    particles that are moved apart are tried at once."""
+    m, ref = (_model((96, 64), TOUCHING, s) for s in ("auto", "stream"))
+    calls = [_launches(lib, m, 1) for _ in range(1 + 63 + 1 + 127 + 1)]
+    assert [k for k, n in enumerate(calls) if n != 3] == [0, 64, 192]
+    assert all(n == 4 for n in (calls[0], calls[64], calls[192]))
+    for _ in range(len(calls)):
+        ref.step(1)
+    np.testing.assert_array_equal(m.distributions, ref.distributions)
+    s = m.particle_states()[1]
+    s.position[0] = 30.0
+    assert lib.lbm_set_particle(m.handle, 2, C.byref(s)) == 0
+    assert _launches(lib, m, 30) == 1
