@@ -19,6 +19,7 @@
 #include <cstring>
 #include <atomic>
 #include <charconv>
+#include <climits>
 #include <chrono>
 #include <thread>
 #include <unordered_map>
@@ -65,6 +66,9 @@ constexpr size_t kMappedReadBytes = size_t(4) << 20;
 // ticks (one to a few recomputations of every tick repay the build), shorter
 // ones launch them directly.
 constexpr int kAdjointGraphTicks = 256;
+// Forward ticks of lbm_adjoint between two looks at the error word (each waits
+// for the device, about 10 us); the particle update keeps the tick.
+constexpr int kAdjointCheckTicks = 256;
 
 }  // namespace
 
@@ -167,6 +171,7 @@ struct lbm_handle {
     double* d_trj = nullptr;
     long long trj_cap = 0, trj_read = 0;
     ParticleDev* d_rec = nullptr;  // particle history of a running lbm_adjoint
+    int* d_rec_err = nullptr;      // and its first tick in error (ParticleArgs::first_err)
     // asynchronous writer of fluid snapshots (lbm_write_fluid_csv)
     std::thread writer;
     std::string writer_err;
@@ -750,6 +755,7 @@ ParticleArgs particle_args(const lbm_handle* h, int mode, int pid, int src = -1)
     a.trj = h->d_trj;
     a.trj_cap = h->trj_cap;
     a.rec = h->d_rec;
+    a.first_err = h->d_rec_err;
     a.fint = h->inter.empty() ? nullptr : h->d_fint;
     return a;
 }
@@ -1341,6 +1347,12 @@ int check_device_error(lbm_handle* h, bool allocate = true) {
     int err = 0;
     CUDA_TRY(h, read_small(&err, h->d_err, sizeof(int), h->stream, allocate));
     if (err == 0) return LBM_OK;
+    long long tick = h->tick;
+    if (h->d_rec_err) {  // lbm_adjoint looks at the word once in many ticks
+        int first = 0;
+        CUDA_TRY(h, read_small(&first, h->d_rec_err, sizeof(int), h->stream));
+        if (first < INT_MAX) tick = first;
+    }
     h->res_ready = false;  // a launch that gave up may have left its masks set
     CUDA_TRY(h, cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -1350,7 +1362,7 @@ int check_device_error(lbm_handle* h, bool allocate = true) {
     if (err & kErrNumeric)
         return set_err(h, LBM_ERR_NUMERIC,
                        "non-finite or negative density on the device (the simulation diverged near tick " +
-                           std::to_string(h->tick) + ")");
+                           std::to_string(tick) + ")");
     return set_err(h, LBM_ERR_STATE, "unknown device error word " + std::to_string(err));
 }
 
@@ -3487,6 +3499,7 @@ struct AdjointRun {
     int lcur = 0;  // lam[lcur]: adjoint of the populations at the current tick
     unsigned link_ctas = 0;
     bool graphs = false;  // long runs replay graphs, short ones launch their ticks
+    long long unchecked = 0;  // forward ticks since the error word was read
     bool begun = false;
 };
 
@@ -3589,8 +3602,11 @@ int advance(AdjointRun& R, long long k) {
         R.have[++h->tick] = 1;
     }
     R.forward += k;
+    R.unchecked += k;
     CUDA_TRY(h, cudaGetLastError());
-    return k >= kModelGraphTicks ? check_device_error(h) : LBM_OK;  // a long segment that diverged ends the run
+    if (R.unchecked < kAdjointCheckTicks) return LBM_OK;
+    R.unchecked = 0;
+    return check_device_error(h);
 }
 
 // backward step of tick n; the device holds the state at tick n, and the
@@ -3746,10 +3762,13 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
     if (!rc) rc = take(&dmu, sizeof(double) * h->N);
     if (!rc) rc = take(&partial, part_bytes);
     if (!rc) rc = take(&st, sizeof(AdjState));
+    if (!rc) rc = take(&h->d_rec_err, sizeof(int));
+    const int none = INT_MAX;
     if (!rc) rc = take(&h->d_rec, rec_bytes);
     if (!rc && (cudaMemsetAsync(R.lam[0], 0, lam_bytes, h->stream) != cudaSuccess ||
                 cudaMemsetAsync(dmu, 0, sizeof(double) * h->N, h->stream) != cudaSuccess ||
                 cudaMemsetAsync(st, 0, sizeof(AdjState), h->stream) != cudaSuccess ||
+                cudaMemcpyAsync(h->d_rec_err, &none, sizeof(int), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
                 cudaMemcpyAsync(h->d_rec, h->d_parts, sizeof(ParticleDev), cudaMemcpyDeviceToDevice, h->stream) !=
                     cudaSuccess))
         rc = set_err(h, LBM_ERR_CUDA, "memset failed");
@@ -3823,6 +3842,7 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
     dev_free(partial);
     dev_free(st);
     dev_free(h->d_rec);
+    dev_free(h->d_rec_err);
     drop_graphs(h);  // they write the history
     h->device_bytes -= held + R.snap_bytes * R.extra.size();
     if (rc) return rc;

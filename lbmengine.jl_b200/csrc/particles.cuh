@@ -10,6 +10,7 @@
 // kept as a list of (fluid cell, direction mask) entries that is rebuilt only
 // when the intervals change; a sub-node move leaves both untouched.
 #pragma once
+#include <climits>
 #include "kernels.cuh"
 
 namespace lbm {
@@ -45,6 +46,7 @@ struct ParticleArgs {
                        // velocity after each tick's update), or null
     long long trj_cap;
     ParticleDev* rec;    // the particle's record after each tick, [ticks + 1] (one particle), or null
+    int* first_err;      // with rec: the tick whose update was the first to find the error word set (INT_MAX: none)
     const double* fint;  // [nparts][3] forces of the particle interactions (interactions.cuh), or null
 };
 
@@ -59,6 +61,7 @@ __device__ __forceinline__ void store_record(const ParticleArgs& a, int p, const
         dst[k] = src[k];
         if (rec) rec[k] = src[k];
     }
+    if (rec && threadIdx.x == 0 && *(volatile const int*)a.err) atomicCAS(a.first_err, INT_MAX, P.rec_tick);
 }
 
 // publish particle p's solid box for the far/near split of the bulk pass
