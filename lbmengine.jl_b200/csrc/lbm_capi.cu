@@ -3764,12 +3764,24 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
     if (!rc) rc = take(&st, sizeof(AdjState));
     if (!rc) rc = take(&h->d_rec_err, sizeof(int));
     const int none = INT_MAX;
-    if (!rc) rc = take(&h->d_rec, rec_bytes);
+    // the particle history grows with the run: where it does not fit beside the rest, the kernels keep it in
+    // pinned host memory, a record a tick
+    void* host_rec = nullptr;
+    if (!rc && take(&h->d_rec, rec_bytes) != LBM_OK) {
+        if (cudaHostAlloc(&host_rec, rec_bytes, cudaHostAllocMapped) == cudaSuccess) {
+            h->d_rec = static_cast<ParticleDev*>(host_rec);  // one address space
+            h->err.clear();
+        } else {
+            cudaGetLastError();
+            host_rec = nullptr;
+            rc = LBM_ERR_OOM;
+        }
+    }
     if (!rc && (cudaMemsetAsync(R.lam[0], 0, lam_bytes, h->stream) != cudaSuccess ||
                 cudaMemsetAsync(dmu, 0, sizeof(double) * h->N, h->stream) != cudaSuccess ||
                 cudaMemsetAsync(st, 0, sizeof(AdjState), h->stream) != cudaSuccess ||
                 cudaMemcpyAsync(h->d_rec_err, &none, sizeof(int), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
-                cudaMemcpyAsync(h->d_rec, h->d_parts, sizeof(ParticleDev), cudaMemcpyDeviceToDevice, h->stream) !=
+                cudaMemcpyAsync(h->d_rec, h->d_parts, sizeof(ParticleDev), cudaMemcpyDefault, h->stream) !=
                     cudaSuccess))
         rc = set_err(h, LBM_ERR_CUDA, "memset failed");
     drop_graphs(h);  // the ticks below also write the history
@@ -3823,7 +3835,7 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
             rec.resize(T + 1);
             // on the handle's stream: a plain cudaMemcpy would not wait for it
             if (cudaMemcpyAsync(&G, st, sizeof(G), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
-                cudaMemcpyAsync(rec.data(), h->d_rec, rec_bytes, cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
+                cudaMemcpyAsync(rec.data(), h->d_rec, rec_bytes, cudaMemcpyDefault, h->stream) != cudaSuccess ||
                 cudaStreamSynchronize(h->stream) != cudaSuccess)
                 rc = set_err(h, LBM_ERR_CUDA, "read-back failed");
             else
@@ -3841,6 +3853,10 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
     dev_free(dmu);
     dev_free(partial);
     dev_free(st);
+    if (host_rec) {
+        cudaFreeHost(host_rec);
+        h->d_rec = nullptr;
+    }
     dev_free(h->d_rec);
     dev_free(h->d_rec_err);
     drop_graphs(h);  // they write the history

@@ -101,3 +101,31 @@ def test_small_model_at_the_limit_steps_in_stream_order(lib, walls, extra):
             assert launches(lib, small) == 3 * n
     assert small.info().device_bytes == before
     np.testing.assert_array_equal(small.distributions, ref.distributions)
+
+
+def test_gradient_of_many_ticks_needs_no_more_device_memory(lib):
+    """The device memory that six ticks' gradient fits into does for a thousand: the particle's history goes to host
+    memory where the rest fills the limit, with the same result."""
+    from lbmengine.adjoint import swimming_speed_gradient
+
+    def gradient(ticks):
+        m = _swimmer(storage="f32")
+        out = swimming_speed_gradient(m, ticks, (ticks - 2, ticks), snapshots=3)
+        m.close()
+        return out
+
+    base = _swimmer().info().device_bytes
+    low, high = base, base + (1 << 26)  # refused; enough
+    while high - low > 64:
+        mid = (low + high) // 2
+        with limit(lib, mid):
+            try:
+                gradient(6)
+                high = mid
+            except capi.LbmError as e:
+                assert e.code == capi.LBM_ERR_OOM
+                low = mid
+    want = gradient(1000)
+    with limit(lib, high):
+        got = gradient(1000)
+    assert got.value == want.value and got.grad == want.grad
