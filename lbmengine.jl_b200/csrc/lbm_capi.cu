@@ -960,17 +960,23 @@ int prepare_tick(lbm_handle* h) {
 
 // ---- many ticks per launch (resident.cuh) -----------------------------------
 
-// Grids that run resident, in nodes.  With a particle a resident tick takes
-// 3.4-4.6 us up to 2^17 nodes (the particle's chain) where the stream schedule
-// takes 9.2-11 us; from there on both grow with the grid, the stream schedule
-// more slowly (it moves four nodes per thread): 8.9 against 11.2 us at 724^2
-// FP32, 11.7 against 14.1 at 1024 x 512 FP64, 16.3 against 12.7 at 1024^2.  With
-// walls alone 2.6 against 5.0 us at 13,000 nodes, 6.1 against 6.9 at 255,000.
-// Plain fluid needs no barrier beside the tick itself: 2.1 against 2.2 us on
-// one cluster, and the stream schedule is level or faster beyond.
-constexpr long long kResidentNodesPart = 1ll << 19;
-constexpr long long kResidentNodesWalls = 1ll << 18;
-constexpr long long kResidentNodesFluid = (kResMaxCluster - 1) * kResThreads;
+// Grids that run resident, in nodes.  Calls of 512 ticks, us per tick, resident / stream:
+//   particle  FP32 5.8 / 9.1 at 250,000 nodes, 9.0 / 9.9 at 490,000; FP64 11.3 / 13.3 at 490,000
+//   walls     FP32 in rows for the vector bulk kernel 4.8 / 5.4 at 160,000 nodes, 5.0 / 4.6 at 193,600, in
+//             other rows 5.2 / 6.5 at 216,200; FP64 7.2 / 8.1 at 261,000
+//   both      FP32 in such rows 7.9 / 9.8 at 360,000, 10.2 / 9.6 at 490,000, in other rows 10.0 / 11.7 at 523,000;
+//             FP64 12.2 / 13.3 at 490,000
+//   neither   (one cluster) FP32 2.12 / 2.20 at 4,096, 2.15 / 2.20 at 7,569; FP64 2.53 / 2.49 and 2.57 / 2.37
+// A first call too long for direct launches is exempt up to kResidentFirst
+// ticks: the stream schedule would build its graphs in it, about 250 us.
+constexpr int64_t kResidentFirst = 512;
+long long resident_nodes(const lbm_handle* h, int64_t nsteps) {
+    const bool first = h->calls == 0 && nsteps > kFirstCallDirectTicks && nsteps <= kResidentFirst;
+    const bool f32_rows = h->storage == ST_F32 && h->n[0] % 4 == 0 && !first;
+    if (!h->hparts.empty()) return h->has_walls && f32_rows ? 7ll << 16 : 1ll << 19;
+    if (h->has_walls) return f32_rows ? 5ll << 15 : 1ll << 18;
+    return h->storage == ST_F32 || first ? (kResMaxCluster - 1) * kResThreads : 0;
+}
 constexpr int64_t kResidentTicks = 4096;  // ticks per launch
 // A launch ends early where particles are close, and they stay so for a while:
 // the next kResidentHold ticks run in stream order without another attempt,
@@ -1073,10 +1079,10 @@ int resident_buffers(lbm_handle* h) {
     return LBM_OK;
 }
 
-// whether lbm_step runs resident; then the buffers are there and the jobs current
-bool use_resident(lbm_handle* h) {
+// whether a call of nsteps ticks runs resident; then the buffers are there and the jobs current
+bool use_resident(lbm_handle* h, int64_t nsteps) {
     if (!h->auto_schedule || h->bulk_kind != LBM_BULK_AUTO || h->profiling >= 2 || !resident_applies(h) ||
-        h->N > (!h->hparts.empty() ? kResidentNodesPart : (h->has_walls ? kResidentNodesWalls : kResidentNodesFluid)))
+        h->N > resident_nodes(h, nsteps))
         return false;
     if (h->res_ctas < 0) {
         // one node per thread, and a CTA per particle: a cluster where that
@@ -2070,7 +2076,7 @@ int lbm_step(lbm_handle* h, int64_t nsteps) {
     if (!h) return set_err(h, LBM_ERR_INVALID, "null handle");
     if (nsteps < 0) return set_err(h, LBM_ERR_INVALID, "ticks must be non-negative");
     BIND(h);
-    const bool resident = h->res_hold <= 0 && use_resident(h);
+    const bool resident = h->res_hold <= 0 && use_resident(h, nsteps);
     const bool first = h->calls++ == 0;
     int64_t done = 0, launches = 0;
     bool direct = false;

@@ -91,3 +91,16 @@ def test_close_particles_do_not_pay_for_an_attempt_per_call(lib):
     s.position[0] = 30.0
     assert lib.lbm_set_particle(m.handle, 2, C.byref(s)) == 0
     assert _launches(lib, m, 30) == 1
+
+
+@pytest.mark.parametrize("n,parts,walls,storage,resident", [
+    ((64, 64), [], False, "f32", True), ((64, 64), [], False, "f64", False), ((87, 87), [], False, "f64", False),
+    ((400, 400), [], True, "f32", True), ((440, 440), [], True, "f32", False), ((441, 440), [], True, "f32", True),
+    ((440, 440), [], True, "f64", True), ((600, 600), ONE, True, "f32", True), ((700, 700), ONE, True, "f32", False),
+    ((701, 700), ONE, True, "f32", True), ((700, 700), ONE, False, "f32", True), ((700, 700), ONE, True, "f64", True)])
+def test_grids_on_both_sides_of_the_limits(lib, n, parts, walls, storage, resident):
+    """Larger grids, and FP64 fluid alone, are faster in stream order; a first call of some length runs as one launch
+    all the same, instead of building the stream schedule's graphs."""
+    m = _model(n, parts, walls=walls, storage=storage)
+    in_order = 50 * (1 + bool(parts or walls) + bool(parts))
+    assert [_launches(lib, m, 50) for _ in range(2)] == [1, 1 if resident else in_order]
