@@ -977,6 +977,20 @@ long long resident_nodes(const lbm_handle* h, int64_t nsteps) {
     if (h->has_walls) return f32_rows ? 5ll << 15 : 1ll << 18;
     return h->storage == ST_F32 || first ? (kResMaxCluster - 1) * kResThreads : 0;
 }
+// Calls from how many ticks on run resident: a launch costs about 10 us more than
+// a graph replay (its prologue, two memsets for a grid; with several particles a
+// blocking read) and gains some microseconds per tick.  us per call, resident /
+// stream (FP32; FP64 alike):
+//   fluid 64^2                    2 ticks 26 / 19, 4 26 / 25, 8 38.6 / 38.6, 10 39 / 42
+//   walls, 11,000 nodes           1 28 / 17, 2 29 / 27, 3 29 / 28, 5 33 / 39; 99,000 nodes 4 41 / 37, 8 53 / 51, 10 57 / 68
+//   one particle, r = 3           1 29 / 25, 2 33 / 39; r = 14 2 41 / 39, 3 41 / 52; r = 28 3 53 / 52, 4 54 / 50, 5 65 / 65, 6 67 / 77
+//   eight particles, 11,520 nodes 1 42 / 25, 3 52 / 52, 5 62 / 66; 490,000 nodes 5 87 / 75, 10 131 / 139
+int64_t resident_min_ticks(const lbm_handle* h) {
+    const size_t np = h->hparts.size();
+    if (np > 1) return h->N <= 1 << 18 ? 5 : 10;
+    if (np == 1) return list_chunks(h) == 1 ? 2 : list_chunks(h) <= 4 ? 3 : 5;
+    return h->has_walls && h->N <= 1 << 16 ? 3 : 10;
+}
 constexpr int64_t kResidentTicks = 4096;  // ticks per launch
 // A launch ends early where particles are close, and they stay so for a while:
 // the next kResidentHold ticks run in stream order without another attempt,
@@ -1082,7 +1096,7 @@ int resident_buffers(lbm_handle* h) {
 // whether a call of nsteps ticks runs resident; then the buffers are there and the jobs current
 bool use_resident(lbm_handle* h, int64_t nsteps) {
     if (!h->auto_schedule || h->bulk_kind != LBM_BULK_AUTO || h->profiling >= 2 || !resident_applies(h) ||
-        h->N > resident_nodes(h, nsteps))
+        h->N > resident_nodes(h, nsteps) || nsteps < resident_min_ticks(h))
         return false;
     if (h->res_ctas < 0) {
         // one node per thread, and a CTA per particle: a cluster where that

@@ -22,10 +22,10 @@ def _model(parts, walls=False):
 
 
 @pytest.mark.parametrize("parts,walls", [(0, True), (1, False), (1, True), (2, False)])
-@pytest.mark.parametrize("ticks", [3, 9000])  # one launch; three
+@pytest.mark.parametrize("ticks", [10, 9000])  # one launch; three
 def test_barrier_gives_up_with_timeout(lib, tmp_path, parts, walls, ticks):
     m = _model(parts, walls)
-    m.step(2)
+    m.step(10)
     path = str(tmp_path / "state.lbm")
     m.save_state(path)
     assert lib.lbm_set_wait_limit(m.handle, 2000, 1) == 0
@@ -34,9 +34,9 @@ def test_barrier_gives_up_with_timeout(lib, tmp_path, parts, walls, ticks):
     assert e.value.code == capi.LBM_ERR_TIMEOUT
     assert lib.lbm_set_wait_limit(m.handle, 1 << 22, 0) == 0
     m.load_state(path)
-    m.step(3)
+    m.step(10)
     ref = _model(parts, walls)
-    ref.step(5)
+    ref.step(20)
     np.testing.assert_array_equal(m.distributions, ref.distributions)
     for p, q in zip(m.particle_states(), ref.particle_states()):
         assert list(p.position) == list(q.position) and list(p.velocity) == list(q.velocity)
@@ -48,7 +48,7 @@ def test_recovery_without_new_limits(lib, tmp_path):
     """The masks of a launch that gave up are cleared by the error itself: the same short limit, which ordinary
     waits of this grid may exceed or not, is kept, and only the state is loaded again."""
     m = _model(1)
-    m.step(1)
+    m.step(5)
     path = str(tmp_path / "state.lbm")
     m.save_state(path)
     assert lib.lbm_set_wait_limit(m.handle, 1, 0) == 0
@@ -62,5 +62,5 @@ def test_recovery_without_new_limits(lib, tmp_path):
     m.load_state(path)
     m.step(20)
     ref = _model(1)
-    ref.step(21)
+    ref.step(25)
     np.testing.assert_array_equal(m.distributions, ref.distributions)
