@@ -1000,19 +1000,41 @@ __device__ __forceinline__ void bulk_v4_tile(const StepArgs& a, long long tile, 
         y, z, dither, keep);
 }
 
-// Resident threads per SM the vector bulk kernels are compiled for: a D2Q9
-// thread holds 36 populations and fits 64 registers (32 warps per SM).  The 3D
-// sets hold 60 to 108 and must not spill: with the packed collision D3Q15 and
-// D3Q19 take 128 registers (16 warps), D3Q15 with 2-byte storage 96 (20 warps),
-// D3Q27 168 (12 warps).  D3Q19 FP16 compiled for 20 warps spilled 44 bytes per
-// thread and its 128^3 pass took 35.9 us instead of 28.7.  The scalar
-// collision (X2 = false) fits 20 warps with 2-byte storage (14 for D3Q27).
+// Resident threads per SM the vector bulk kernels are compiled for, by the
+// registers that their populations (36 values per D2Q9 thread, 60 to 108 in 3D)
+// leave free of spills or nearly so: D2Q9 64 registers (32 warps per SM; the
+// packed 2-byte forms spill 8-20 bytes in them, FP32 BGK 28, and 72 registers
+// with fewer warps took 20 % longer on grids beyond L2), D3Q15 and D3Q19 128 (16
+// warps), D3Q15 with 2-byte storage 96 (20 warps, 0-8 bytes), D3Q27 168 (12
+// warps; BGK with stochastic rounding 16 bytes).  D3Q19 FP16 compiled for 20
+// warps spilled 44 bytes per thread and its 128^3 pass took 35.9 us instead of
+// 28.7.  The scalar collision (X2 = false) fits 20 warps with 2-byte storage (14
+// for D3Q27).
 template <class L, int ST = ST_F32, bool SR = false, bool X2 = false>
 constexpr int bulk_threads_per_sm() {
     if (L::Q <= 9) return 1024;
     if (Store<ST>::bytes != 2) return L::Q > 19 ? 384 : 512;
     if (X2) return L::Q > 19 ? 384 : (L::Q == 19 ? 512 : 640);
     return L::Q > 19 ? 448 : 640;
+}
+
+// Whether CTAs of B threads take the packed collision.  512 threads leave 128
+// registers, into which the packed D3Q27 forms spill 50 to 156 bytes.  With
+// 2-byte storage TRT loses by it (FP16, packed / scalar: 1200 x 40 x 40 nodes
+// 82 / 60 us, 516 x 64 x 64 84 / 64, 28 x 100 x 100 15.6 / 13.5); BGK (61.5 / 63.5 with
+// nearest, 64.3 / 64.4 with stochastic rounding) and FP32 (88 / 89) do not.
+template <class L, int ST, bool TRT, int B>
+constexpr bool bulk_packed() {
+    return !(B == 512 && L::Q > 19 && Store<ST>::bytes == 2 && TRT);
+}
+// D2Q9 FP32 BGK loses the packed form's gain to its spills where memory is the
+// bound: population buffers beyond L2 take the scalar one (packed / scalar:
+// 2048^2 48.6 / 47.5 us, 1920 x 2200 49.2 / 48.0, 1800^2 (117 MB) 39.0 / 38.9,
+// 1024^2 12.4 / 13.0, 768 x 700 8.2 / 9.0).
+constexpr long long kL2Bytes = 126ll << 20;
+template <class L, int ST, bool TRT>
+constexpr bool bulk_scalar_beyond_l2() {
+    return L::Q <= 9 && ST == ST_F32 && !TRT;
 }
 
 // the vector bulk pass over all tiles, one CTA of B threads per tile
@@ -1022,8 +1044,8 @@ constexpr int bulk_threads_per_sm() {
 // 128^3 FP32 population buffer): a share of each tick's reads comes from L2
 // instead of HBM (the 128^3 FP32 tick 55.2 -> 51.3 us).  The result does not
 // depend on the order.
-template <class L, int ST, bool TRT, int B, bool SR>
-__global__ void __launch_bounds__(B, bulk_threads_per_sm<L, ST, SR, true>() / B) k_bulk_v4(const StepArgs a) {
+template <class L, int ST, bool TRT, int B, bool SR, bool X2 = bulk_packed<L, ST, TRT, B>()>
+__global__ void __launch_bounds__(B, bulk_threads_per_sm<L, ST, SR, X2>() / B) k_bulk_v4(const StepArgs a) {
     __shared__ float s_ex[x_moving_dirs<L>()][B];
     grid_dep_trigger();  // the fix-up may start its stores-free part during the last wave
     const long long tiles = (long long)a.vnt1 * a.g.n[2];
@@ -1032,8 +1054,8 @@ __global__ void __launch_bounds__(B, bulk_threads_per_sm<L, ST, SR, true>() / B)
     // none, 50.5 with two fifths, 49.4 with three, 50.2 with four, 51.6 with
     // all); the issue-bound 2-byte passes measured slower with it
     const bool keep = Store<ST>::bytes == 4 && (long long)blockIdx.x * 5 >= tiles * 2;
-    bulk_v4_tile<L, ST, TRT, B, SR, true>(a, a.reverse ? tiles - 1 - (long long)blockIdx.x : (long long)blockIdx.x, s_ex,
-                                    keep);
+    bulk_v4_tile<L, ST, TRT, B, SR, X2>(a, a.reverse ? tiles - 1 - (long long)blockIdx.x : (long long)blockIdx.x, s_ex,
+                                        keep);
 }
 
 // periodic intervals [a0, a0+la) and [b0, b0+lb) of an axis of n nodes meet

@@ -110,15 +110,24 @@ struct OpsImpl {
         k_links_write<L><<<(unsigned)(nparts * bpp), kLinkBlock, 0, s>>>(a, bpp, counts);
     }
     static constexpr bool kTwo = Store<ST>::bytes == 2;  // stochastic variants exist for 2-byte storage
+    template <int B, bool SR>
+    static void bulk_v4_block(const StepArgs& a, unsigned g, cudaStream_t s) {
+        if constexpr (bulk_scalar_beyond_l2<L, ST, TRT>())
+            if (a.g.N * L::Q * Store<ST>::bytes > kL2Bytes) {
+                k_bulk_v4<L, ST, TRT, B, SR, false><<<g, B, 0, s>>>(a);
+                return;
+            }
+        k_bulk_v4<L, ST, TRT, B, SR><<<g, B, 0, s>>>(a);
+    }
     template <bool SR>
     static void bulk_v4_sr(const StepArgs& a, long long tiles, int block, cudaStream_t s) {
         const unsigned g = (unsigned)tiles;
-        if (block <= 32) k_bulk_v4<L, ST, TRT, 32, SR><<<g, 32, 0, s>>>(a);
-        else if (block <= 64) k_bulk_v4<L, ST, TRT, 64, SR><<<g, 64, 0, s>>>(a);
-        else if (block <= 96) k_bulk_v4<L, ST, TRT, 96, SR><<<g, 96, 0, s>>>(a);
-        else if (block <= 128) k_bulk_v4<L, ST, TRT, 128, SR><<<g, 128, 0, s>>>(a);
-        else if (block <= 256) k_bulk_v4<L, ST, TRT, 256, SR><<<g, 256, 0, s>>>(a);
-        else k_bulk_v4<L, ST, TRT, 512, SR><<<g, 512, 0, s>>>(a);
+        if (block <= 32) bulk_v4_block<32, SR>(a, g, s);
+        else if (block <= 64) bulk_v4_block<64, SR>(a, g, s);
+        else if (block <= 96) bulk_v4_block<96, SR>(a, g, s);
+        else if (block <= 128) bulk_v4_block<128, SR>(a, g, s);
+        else if (block <= 256) bulk_v4_block<256, SR>(a, g, s);
+        else bulk_v4_block<512, SR>(a, g, s);
     }
     static void bulk_v4(const StepArgs& a, long long tiles, int block, cudaStream_t s) {
         if constexpr (ST != ST_F64) {
