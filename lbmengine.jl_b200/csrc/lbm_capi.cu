@@ -878,13 +878,25 @@ int slot_list(lbm_handle* h) {
 //          192^3 FP32, 1 of r = 40 228 / 242;  96^3 FP32, 27 of r = 6 35.7 / 36.8
 //          64^3  FP32, 64 of r = 6 (704 chunks) 44.7 / 37.4;  64 of r = 4 (320 chunks) 25.7 / 30.4
 //   D2Q9   2048^2 FP32, 250 of r = 20 103 / 66;  1024^2 FP32, 250 of r = 8 28.5 / 23.5
+// D3Q27's list CTAs hold more registers and memory, and hold the bulk pass up
+// where there are few of them beside a long pass, with FP64 storage always:
+//   D3Q27  FP32  27 of r = 6 (297 chunks) 96^3 53.5 / 61.2, 128^3 98.9 / 96.4, 160^3 168 / 193;  160^3, 2 of r = 25 (380) 171 / 189
+//                64 of r = 5 (512) 96^3 65.0 / 61.6;  128^3, 8 of r = 16 115 / 94;  160^3, 64 of r = 8 210 / 203
+//          FP16  27 of r = 6 128^3 61.5 / 63.9, 160^3 105 / 93.6;  160^3, 2 of r = 25 109 / 98;  128^3, 64 of r = 6 77.4 / 63.1
+//          FP64  128^3, 27 of r = 6 172 / 287;  96^3, 64 of r = 5 107 / 114;  160^3, 64 of r = 8 359 / 418
+// There: none with FP64, else one and a half waves, or with 2-byte storage a
+// bulk pass of two particle updates.
 constexpr long long kFixWave = 296;
 bool many_chunks(const lbm_handle* h) {
     const long long np = (long long)h->hparts.size(), chunks = np * list_chunks(h);
     if (!fixup_walk(h) || chunks <= kFixWave) return false;
     double r = 0;
     for (const auto& P : h->hparts) r = std::max(r, P.radius / h->dx);
-    return bulk_us(h) >= (h->dims == 3 ? 18.0 + 0.095 * r * r : 10.0) || (chunks >= 2 * kFixWave && np >= 8);
+    const double update = h->dims == 3 ? 18.0 + 0.095 * r * r : 10.0;
+    if (h->q == 27 && (h->storage == ST_F64 || (2 * chunks <= 3 * kFixWave &&
+                                                 (h->storage == ST_F32 || bulk_us(h) < 2.0 * update))))
+        return false;
+    return bulk_us(h) >= update || (chunks >= 2 * kFixWave && np >= 8);
 }
 bool fixup_beside(const lbm_handle* h) { return h->profiling < 2 && h->slot_cap > 0 && many_chunks(h); }
 
