@@ -1159,7 +1159,7 @@ int resident_ticks(lbm_handle* h, int64_t nsteps, int64_t* ran, int64_t* launche
         r.cap_slots = (int)caps.slots;
         r.cap_box = (int)caps.box;
         r.err = h->d_err;
-        r.spin_limit = h->spin_limit;
+        r.spin_limit = (int)h->spin_limit;
         r.wait_extra = (unsigned)h->wait_extra;
         if (h->res_cluster == 0) {
             r.bar = reinterpret_cast<unsigned*>(h->d_rsync);

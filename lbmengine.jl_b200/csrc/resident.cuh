@@ -68,7 +68,7 @@ struct ResidentArgs {
     unsigned* bar;       // grid barrier: counter (zero at launch) and the phase the launch ends at (all
                          // ones at launch); null: cluster barrier
     int* err;            // of the grid barrier
-    long long spin_limit;  // polls before a wait at the grid barrier gives up (2^22: about a second)
+    int spin_limit;        // polls before a wait at the grid barrier gives up (2^22: about a second)
     unsigned wait_extra;   // test knob: added to the count it waits for
 };
 
@@ -113,8 +113,8 @@ struct ResidentBarrier {
     int* err;
     unsigned phase;     // phases completed
     unsigned ctas;
-    long long limit;    // polls of a wait
-    unsigned extra;
+    int limit;          // polls of a wait
+    unsigned goal;      // arrivals that the last wait waited for (at first: wait_extra)
     __device__ __forceinline__ void arrive(bool stop = false) {
         if (ctr) {
             if (threadIdx.x == kResThreads - 32) {
@@ -141,13 +141,13 @@ struct ResidentBarrier {
             cluster_wait();
             return kGoOn;
         }
+        goal += ctas;
         __shared__ int s_state;
         if (threadIdx.x == 0) {
-            int state = kGoOn;
-            long long it = 0;
+            int state = kGoOn, it = 0;
             while (true) {
                 const unsigned v = load(ctr);
-                if ((v & 0x7fffffffu) >= phase * ctas + extra) {
+                if ((v & 0x7fffffffu) >= goal) {
                     if ((v & 0x80000000u) && load(ctr + 1) <= phase) state = kStop;
                     break;
                 }
@@ -735,7 +735,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             B.cu[l] = ci0 * up[0] + ci1 * up[1] + ci2 * up[2];
         }
     };
-    const int ninter = boundary && J.in.nitems > 0 ? J.in.coff[p + 1] - J.in.coff[p] : 0;
+    // what the tick loop wants of the job, in registers: behind the barrier's
+    // acquire every read of it would go to L2 again
+    const bool inter = J.in.nitems > 0;
+    const int inter0 = boundary && inter ? J.in.coff[p] : 0, ninter = boundary && inter ? J.in.coff[p + 1] - inter0 : 0;
+    const int* const inter_cent = J.in.cent;
+    const InterItem* const inter_items = J.in.items;
+    double* const positions = J.pos;
     if (boundary) {
         const unsigned long long* from = reinterpret_cast<const unsigned long long*>(s_pa.parts + p);
         for (int k = tid; k < (int)(sizeof(ParticleDev) / 8); k += kResThreads)
@@ -787,12 +793,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                 for (int j = 1; j < Q; ++j)
                     if (mask >> j & 1u) B.gi[l++] = g[L::opp(j)] * R(a.inv_scale);
             }
-            if (J.in.nitems > 0) {  // interactions: the positions at the start of the tick (interactions.cuh)
-                const double* pos = J.pos + (size_t)(t & 1) * 3 * np;
+            if (inter) {  // interactions: the positions at the start of the tick (interactions.cuh)
+                const double* pos = positions + (size_t)(t & 1) * 3 * np;
                 if (tid >= kResThreads - kResMaxInter && tid - (kResThreads - kResMaxInter) < ninter) {
                     const int q = tid - (kResThreads - kResMaxInter);
-                    const int c = J.in.cent[J.in.coff[p] + q];
-                    const InterItem it = J.in.items[c >> 3];
+                    const int c = inter_cent[inter0 + q];
+                    const InterItem it = inter_items[c >> 3];
                     double R1[3], R2[3], R3[3], out[9];
                     for (int k = 0; k < 3; ++k) {
                         R1[k] = __ldcg(pos + 3 * it.id1 + k);
@@ -859,11 +865,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                 __syncthreads();
             }
             if (warp == 0)
-                resident_translate<D>(s_pa, sP, s_keep, s_part, nch, lane, J.in.nitems > 0 ? s_fint : nullptr, &s_new);
+                resident_translate<D>(s_pa, sP, s_keep, s_part, nch, lane, inter ? s_fint : nullptr, &s_new);
             else if (warp == 1)
                 resident_rotate<D>(s_pa, sP, s_part, nch, lane, &s_new);
             __syncthreads();
-            double* next = J.pos + (size_t)((t + 1) & 1) * 3 * np + 3 * p;
+            double* next = positions + (size_t)((t + 1) & 1) * 3 * np + 3 * p;
             if (!s_new.keep) {  // the geometry may change: the full update, and pmask before the barrier
                 const bool changed = particles_core<L, 128>(s_pa, p, sP);
                 __syncthreads();
@@ -879,7 +885,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                     stale = false;
                     __syncthreads();
                 }
-                if (J.in.nitems > 0) {
+                if (inter) {
                     if (tid < D) __stcg(next + tid, s_new.R[tid]);
                     else if (tid < 3) __stcg(next + tid, 0.0);
                     __syncthreads();
