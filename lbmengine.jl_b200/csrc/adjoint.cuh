@@ -353,13 +353,13 @@ __device__ __noinline__ void adjoint_slots(const AdjArgs& a, int x, int y, int z
 
 // CTAs per SM the node kernel is compiled for: as many as its registers (two
 // per FP64 value of lam*, one or two per stored value) allow with a few spilled values at most
-template <class L, int ST>
+template <class L>
 constexpr int adjoint_ctas_per_sm() {
     return L::Q <= 9 ? 5 : (L::Q <= 19 ? 3 : 2);
 }
 
 template <class L, int ST, bool TRT>
-__global__ void __launch_bounds__(kAdjBlock, adjoint_ctas_per_sm<L, ST>()) k_adjoint(const __grid_constant__ AdjArgs a) {
+__global__ void __launch_bounds__(kAdjBlock, adjoint_ctas_per_sm<L>()) k_adjoint(const __grid_constant__ AdjArgs a) {
     using SS = Store<ST>;
     using T = typename SS::T;
     constexpr int Q = L::Q, D = L::D;

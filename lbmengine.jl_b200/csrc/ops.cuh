@@ -16,7 +16,7 @@ struct Ops {
     void (*bulk)(const StepArgs&, unsigned grid, dim3 block, cudaStream_t);
     // early: launch with programmatic stream serialization (the fix-up may
     // start while the kernel before it in the stream still runs)
-    // walk: the chunk-walking kernel (k_fixup_walk), whose grid is fixup_walk_grid
+    // walk: the chunk-walking kernel (k_fixup_walk)
     void (*fixup)(const StepArgs&, unsigned grid, cudaStream_t, bool early, bool walk);
     // beside the bulk pass: the link slots' values to the list, and their stores after it
     void (*fixup_list)(const StepArgs&, unsigned grid, cudaStream_t);
@@ -174,7 +174,7 @@ struct OpsImpl {
         return ResidentBoundary<ST>::bytes(entries, slots, box);
     }
     static void resident_wmask(const unsigned char* wall, const GridDesc& g, unsigned* wmask, cudaStream_t s) {
-        k_resident_wmask<L><<<blocks_for(g.N, 256), 256, 0, s>>>(wall, g, wmask);
+        if constexpr (kResident) k_resident_wmask<L><<<blocks_for(g.N, 256), 256, 0, s>>>(wall, g, wmask);
     }
     static cudaError_t resident(const ResidentArgs& a, int ctas, int csize, cudaStream_t s) {
         if constexpr (kResident) {

@@ -179,12 +179,12 @@ __device__ __forceinline__ void load_pops_l2(const StepArgs& a, int cell, typena
 // except into link slots and wall nodes, and the node's own wall links.
 template <class L, int ST, bool TRT, bool WALLS>
 __device__ __forceinline__ bool resident_node(const StepArgs& a, const unsigned* pmask, const unsigned* wmask,
-                                              int cell, int x, int y, int z, typename Store<ST>::R* g, bool first) {
+                                              int cell, int x, int y, typename Store<ST>::R* g, bool first) {
     using SS = Store<ST>;
     using T = typename SS::T;
     using R = typename SS::R;
     constexpr int Q = L::Q;
-    const int nx = a.g.n[0], ny = a.g.n[1], nz = a.g.n[2];
+    const int nx = a.g.n[0], ny = a.g.n[1];
     const long long N = a.g.N;
     T* dst = static_cast<T*>(a.dst);
     unsigned skip = pmask ? __ldcg(pmask + cell) : 0u;
@@ -204,22 +204,20 @@ __device__ __forceinline__ bool resident_node(const StepArgs& a, const unsigned*
     const R rho = collide_node<L, ST, TRT>(a, cell, true, g);
     const int xs[3] = {x == 0 ? nx - 1 : x - 1, x, x == nx - 1 ? 0 : x + 1};
     const int ys[3] = {y == 0 ? ny - 1 : y - 1, y, y == ny - 1 ? 0 : y + 1};
-    const int zs[3] = {z == 0 ? nz - 1 : z - 1, z, z == nz - 1 ? 0 : z + 1};
 #pragma unroll
     for (int i = 0; i < Q; ++i)
         if (!(skip >> i & 1u))
-            dst[i * N + (xs[L::cx(i) + 1] + nx * (ys[L::cy(i) + 1] + ny * zs[L::cz(i) + 1]))] = SS::enc(g[i], R(1));
+            dst[i * N + (xs[L::cx(i) + 1] + nx * ys[L::cy(i) + 1])] = SS::enc(g[i], R(1));
     if (WALLS && wm) {
 #pragma unroll
         for (int i = 1; i < Q; ++i) {
             if (!(wm >> i & 1u)) continue;  // x + c_i is a wall node: f_j(x) = f*_i(x), j = opp(i)
             const int j = L::opp(i);
-            const int t = xs[L::cx(i) + 1] + nx * (ys[L::cy(i) + 1] + ny * zs[L::cz(i) + 1]);
+            const int t = xs[L::cx(i) + 1] + nx * ys[L::cy(i) + 1];
             if (pmask && (__ldcg(pmask + t) >> j & 1u)) continue;  // also the particle's link: the boundary CTA's
             double v = (double)(g[i] * R(a.inv_scale));
             if (a.uw) {  // moving walls (fluids.jl:168-174)
-                const double dot = -(L::cx(i) * a.uw[t] + L::cy(i) * a.uw[N + t] +
-                                     (L::D == 3 ? L::cz(i) * a.uw[2 * N + t] : 0.0));
+                const double dot = -(L::cx(i) * a.uw[t] + L::cy(i) * a.uw[N + t]);
                 v += 6.0 * (double)rho * dot;
             }
             dst[j * N + cell] = SS::enc((R)v, R(a.scale));
@@ -228,47 +226,33 @@ __device__ __forceinline__ bool resident_node(const StepArgs& a, const unsigned*
     return bad_density(rho);
 }
 
-// Nodes first, first + stride, ... of the grid; D2Q9 two at a time, so that the
-// loads of both are in flight together (the 3D sets fill the registers with one).
+// Nodes first, first + stride, ... of the grid, two at a time, so that the loads
+// of both are in flight together.
 template <class L, int ST, bool TRT, bool WALLS>
 __device__ __forceinline__ void resident_bulk(const StepArgs& a, const unsigned* pmask, const unsigned* wmask,
-                                              int first, int stride, int x, int y, int z, const int* step, bool init) {
+                                              int first, int stride, int x, int y, const int* step, bool init) {
     using R = typename Store<ST>::R;
-    const int nx = a.g.n[0], ny = a.g.n[1], N = (int)a.g.N;
+    const int nx = a.g.n[0], N = (int)a.g.N;
     bool bad = false;
-    auto advance = [&]() {  // (x, y, z) of the node `stride` further on
+    auto advance = [&]() {  // (x, y) of the node `stride` further on
         x += step[0];
         y += step[1];
-        z += step[2];
         if (x >= nx) {
             x -= nx;
             ++y;
         }
-        if (L::D == 3 && y >= ny) {
-            y -= ny;
-            ++z;
-        }
     };
-    if (L::Q <= 9) {
-        for (int cell = first; cell < N; cell += 2 * stride) {
-            const int c2 = cell + stride;
-            const bool two = c2 < N;
-            R g[2][L::Q];
-            load_pops_l2<L, ST>(a, cell, g[0]);
-            load_pops_l2<L, ST>(a, two ? c2 : cell, g[1]);
-            bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, cell, x, y, z, g[0], init);
-            if (!two) break;
-            advance();
-            bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, c2, x, y, z, g[1], init);
-            advance();
-        }
-    } else {
-        for (int cell = first; cell < N; cell += stride) {
-            R g[L::Q];
-            load_pops_l2<L, ST>(a, cell, g);
-            bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, cell, x, y, z, g, init);
-            advance();
-        }
+    for (int cell = first; cell < N; cell += 2 * stride) {
+        const int c2 = cell + stride;
+        const bool two = c2 < N;
+        R g[2][L::Q];
+        load_pops_l2<L, ST>(a, cell, g[0]);
+        load_pops_l2<L, ST>(a, two ? c2 : cell, g[1]);
+        bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, cell, x, y, g[0], init);
+        if (!two) break;
+        advance();
+        bad |= resident_node<L, ST, TRT, WALLS>(a, pmask, wmask, c2, x, y, g[1], init);
+        advance();
     }
     if (bad) atomicOr(a.err, kErrNumeric);
 }
@@ -282,13 +266,10 @@ __global__ void k_resident_wmask(const unsigned char* wall, GridDesc g, unsigned
     if (wall[c]) {
         m = ~0u;
     } else {
-        const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-        const int x = (int)(c % nx), y = (int)((c / nx) % ny), z = (int)(c / ((long long)nx * ny));
+        const int nx = g.n[0], ny = g.n[1], x = (int)(c % nx), y = (int)(c / nx);
 #pragma unroll
         for (int i = 1; i < L::Q; ++i)
-            if (wall[wrap_idx(x + L::cx(i), nx) +
-                     (long long)nx * (wrap_idx(y + L::cy(i), ny) + (long long)ny * wrap_idx(z + L::cz(i), nz))])
-                m |= 1u << i;
+            if (wall[wrap_idx(x + L::cx(i), nx) + (long long)nx * wrap_idx(y + L::cy(i), ny)]) m |= 1u << i;
     }
     wmask[c] = m;
 }
@@ -369,7 +350,7 @@ __device__ __forceinline__ void resident_keep(const ParticleArgs& a, const Parti
 // k), one the rotation.  The new state goes to a ResidentNew; nothing of the
 // record changes before every thread has seen the verdict (keep).
 struct ResidentNew {
-    double v[3], R[3], w[3], e[3], F[3], T[3];
+    double v[2], R[2], e[2], F[2], w, T;
     int moved, alpha, keep;
 };
 // the chunks' sums in the order of particles_core: a butterfly over the lanes of one chunk each (a whole warp)
@@ -427,36 +408,23 @@ template <int D>
 __device__ __forceinline__ void resident_rotate(const ParticleArgs& a, const ParticleDev& P,
                                                 const double (*part)[kPartialStride], int nch, int lane,
                                                 ResidentNew* N) {
-    constexpr int NW = D == 2 ? 1 : 3;
-    double T[3] = {0, 0, 0}, w[3] = {P.w[0], P.w[1], P.w[2]}, e[3] = {P.e[0], P.e[1], P.e[2]};
-#pragma unroll
-    for (int k = 0; k < NW; ++k) T[k] = resident_sum(part, nch, 3 + k, lane);
-    const double dt = a.dt;
+    const double T = resident_sum(part, nch, 3, lane), dt = a.dt;
+    double w = P.w[0], e[3] = {P.e[0], P.e[1], P.e[2]};
     bool alpha = false;
     if (P.rules == 1) {
-#pragma unroll
-        for (int k = 0; k < NW; ++k) {
-            const double dL = dt * T[k];
-            w[k] = w[k] + P.inv_inertia * dL;
-            alpha = alpha || dL != 0.0;
-        }
+        const double dL = dt * T;
+        w = w + P.inv_inertia * dL;
+        alpha = dL != 0.0;
     } else if (P.coupleT) {
-        double Al[3] = {0, 0, 0};
-#pragma unroll
-        for (int k = 0; k < NW; ++k) {
-            Al[k] = T[k] * P.inv_inertia;
-            w[k] = w[k] + dt * Al[k];
-            alpha = alpha || Al[k] != 0.0;
-        }
-        if (P.kind == 1) rotate_direction<D>(w, dt, e);
+        const double Al = T * P.inv_inertia;
+        w = w + dt * Al;
+        alpha = Al != 0.0;
+        if (P.kind == 1) rotate_direction<D>(&w, dt, e);
     }
     if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            N->w[k] = w[k];
-            N->e[k] = e[k];
-            N->T[k] = P.rules == 1 ? dt * T[k] : T[k];
-        }
+        for (int k = 0; k < 2; ++k) N->e[k] = e[k];
+        N->w = w;
+        N->T = P.rules == 1 ? dt * T : T;
         N->alpha = alpha;
     }
 }
@@ -464,7 +432,6 @@ __device__ __forceinline__ void resident_rotate(const ParticleArgs& a, const Par
 template <int D>
 __device__ __forceinline__ void resident_commit(const ParticleArgs& a, int p, ParticleDev& P, const ResidentNew& N,
                                                 int lane) {
-    constexpr int NW = D == 2 ? 1 : 3;
     const bool nv = N.moved || N.alpha;  // getNodeVelocity: the snapshot of the slip velocity
     if (lane < D) {
         P.v[lane] = N.v[lane];
@@ -477,13 +444,13 @@ __device__ __forceinline__ void resident_commit(const ParticleArgs& a, int p, Pa
             P.sE[lane] = N.e[lane];
         }
     }
-    if (lane >= 4 && lane < 4 + NW) {
-        P.w[lane - 4] = N.w[lane - 4];
-        if (nv) P.sW[lane - 4] = N.w[lane - 4];
+    if (lane == 4) {
+        P.w[0] = N.w;
+        if (nv) P.sW[0] = N.w;
     }
     if (lane >= 8 && lane < 11) {
         P.lastF[lane - 8] = lane - 8 < D ? N.F[lane - 8] : 0.0;
-        P.lastT[lane - 8] = N.T[lane - 8];
+        P.lastT[lane - 8] = lane == 8 ? N.T : 0.0;
     }
     if (lane == 11) {
         P.relink = 0;
@@ -503,23 +470,16 @@ __device__ __forceinline__ void resident_commit(const ParticleArgs& a, int p, Pa
 
 // Ladd term and momentum exchange of one slot with the slip velocity's c_i . u
 // already known (ladd_link)
-template <int D>
 __device__ __forceinline__ void resident_exchange(const StepArgs& a, const ParticleDev& P, const int* ci,
                                                   const double* Xc, double gi, double wi, double v, double* acc) {
     const double cs = a.coeff * (wi * (2.0 * a.rho0 + gi + v));
     if (P.coupleF || P.recordF) {
-#pragma unroll
-        for (int k = 0; k < D; ++k) acc[k] += cs * ci[k];
+        acc[0] += cs * ci[0];
+        acc[1] += cs * ci[1];
     }
     if (P.coupleT) {
-        const double r0 = Xc[0] - P.mR[0], r1 = Xc[1] - P.mR[1], r2 = D == 3 ? Xc[2] - P.mR[2] : 0.0;
-        if (D == 2) {
-            acc[3] += cs * (r0 * ci[1] - r1 * ci[0]);
-        } else {
-            acc[3] += cs * (r1 * ci[2] - r2 * ci[1]);
-            acc[4] += cs * (-r0 * ci[2] + r2 * ci[0]);
-            acc[5] += cs * (r0 * ci[1] - r1 * ci[0]);
-        }
+        const double r0 = Xc[0] - P.mR[0], r1 = Xc[1] - P.mR[1];
+        acc[3] += cs * (r0 * ci[1] - r1 * ci[0]);
     }
 }
 
@@ -550,6 +510,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
     using T = typename SS::T;
     using R = typename SS::R;
     constexpr int Q = L::Q, D = L::D;
+    static_assert(D == 2, "a 2D kernel");
     constexpr int kHalves = kResThreads / kResHalf;
     constexpr unsigned kAllDirs = (Q == 32 ? 0u : (1u << Q)) - 2u;
     extern __shared__ __align__(16) unsigned char s_dyn[];
@@ -563,7 +524,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
     __shared__ int s_off[kResMaxChunks + 1];  // first slot of each chunk
     __shared__ int s_wcnt[2], s_stop, s_quit, s_box[6];
     __shared__ int s_nsrc[2];  // source nodes set in each parity's pmask
-    __shared__ int s_lat[4][Q];  // c_i (3) and i of the slot direction j, i = opp(j)
+    __shared__ int s_lat[2][Q];  // c_i of the slot direction j, i = opp(j)
     __shared__ double s_w[Q];
     __shared__ double s_fi[kResMaxInter][3], s_fint[3];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -574,8 +535,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
     for (int j = tid; j < Q; j += kResThreads) {
         s_lat[0][j] = -L::cx(j);
         s_lat[1][j] = -L::cy(j);
-        s_lat[2][j] = -L::cz(j);
-        s_lat[3][j] = L::opp(j);
         s_w[j] = L::w(j);
     }
     const ResidentJob& J = *ra.job;
@@ -595,21 +554,19 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
     const int bulk_ctas = csize - np;
     const bool boundary = rank >= bulk_ctas;
     const int p = rank - bulk_ctas;  // the boundary CTA's particle
-    const int nx = s_a[0].g.n[0], ny = s_a[0].g.n[1], nz = s_a[0].g.n[2];
+    const int nx = s_a[0].g.n[0], ny = s_a[0].g.n[1];
     const long long N = s_a[0].g.N;
     unsigned* const pmask = np > 0 ? J.pmask : nullptr;
     const unsigned* const wmask = J.wmask;
     const int first = rank * kResThreads + tid, stride = bulk_ctas * kResThreads;
-    const int x0 = first % nx, y0 = D == 2 ? first / nx : (first / nx) % ny, z0 = D == 2 ? 0 : first / (nx * ny);
-    const int step[3] = {stride % nx, D == 2 ? stride / nx : (stride / nx) % ny, D == 2 ? 0 : stride / (nx * ny)};
+    const int x0 = first % nx, y0 = first / nx, step[2] = {stride % nx, stride / nx};
     ResidentBoundary<ST> B(s_dyn, ra.cap_entries, ra.cap_slots, ra.cap_box);
     int entries = 0, nch = 0;
     // the source node of slot `item` (the node pushed from by plain streaming)
     auto source = [&](int item) -> int {
         const int cell = B.cell[item >> 5], j = item & 31;
-        const int x = wrap_idx(cell % nx + s_lat[0][j], nx), y = wrap_idx((cell / nx) % ny + s_lat[1][j], ny);
-        const int z = D == 2 ? 0 : wrap_idx(cell / (nx * ny) + s_lat[2][j], nz);
-        return x + nx * (y + ny * z);
+        const int x = wrap_idx(cell % nx + s_lat[0][j], nx), y = wrap_idx(cell / nx + s_lat[1][j], ny);
+        return x + nx * y;
     };
     auto slots = [&]() -> int { return nch > 0 ? s_off[nch] : 0; };
     // pmask of parity b: cleared, and set for the current slots
@@ -724,15 +681,15 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
         const int now = slots();
         for (int l = tid; l < now; l += kResThreads) {
             const int item = B.list[l], e = item >> 5, j = item & 31;
-            const int ci0 = s_lat[0][j], ci1 = s_lat[1][j], ci2 = s_lat[2][j];
-            const double Tc[3] = {coord(e, 0, ci0), coord(e, 1, ci1), D == 3 ? coord(e, 2, ci2) : 0.0};
+            const int ci0 = s_lat[0][j], ci1 = s_lat[1][j];
+            const double Tc[2] = {coord(e, 0, ci0), coord(e, 1, ci1)};
             double up[3];
             if (sP.rules == 1)
                 slip_velocity_cpu<D>(sP.sR, sP.sV, sP.sW, sP.sE, sP.B1, sP.B2, sP.kind, sP.radius,
-                                     2.0 * s_a[0].half_dt, Tc[0], Tc[1], Tc[2], up);
+                                     2.0 * s_a[0].half_dt, Tc[0], Tc[1], 0.0, up);
             else
-                slip_velocity<D>(sP.sR, sP.sV, sP.sW, sP.sE, sP.B1, sP.B2, sP.kind, Tc[0], Tc[1], Tc[2], up);
-            B.cu[l] = ci0 * up[0] + ci1 * up[1] + ci2 * up[2];
+                slip_velocity<D>(sP.sR, sP.sV, sP.sW, sP.sE, sP.B1, sP.B2, sP.kind, Tc[0], Tc[1], 0.0, up);
+            B.cu[l] = ci0 * up[0] + ci1 * up[1];
         }
     };
     // what the tick loop wants of the job, in registers: behind the barrier's
@@ -776,8 +733,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
         const StepArgs& a = s_a[t & 1];
         if (!boundary) {
             const unsigned* pm = pmask ? pmask + (size_t)(t & 1) * N : nullptr;
-            if (walls) resident_bulk<L, ST, TRT, true>(a, pm, wmask, first, stride, x0, y0, z0, step, t < 2);
-            else resident_bulk<L, ST, TRT, false>(a, pm, wmask, first, stride, x0, y0, z0, step, false);
+            if (walls) resident_bulk<L, ST, TRT, true>(a, pm, wmask, first, stride, x0, y0, step, t < 2);
+            else resident_bulk<L, ST, TRT, false>(a, pm, wmask, first, stride, x0, y0, step, false);
             __syncthreads();
             bar.arrive();
         } else {
@@ -822,34 +779,32 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             T* dst = static_cast<T*>(a.dst);
             for (int c0 = 0; c0 < nch; c0 += kHalves) {
                 const int c = c0 + tid / kResHalf;
-                double acc[6] = {0, 0, 0, 0, 0, 0};
+                double acc[4] = {0, 0, 0, 0};  // two force components, (none), the torque
                 if (c < nch) {
                     const int l1 = s_off[c + 1];
                     for (int l = s_off[c] + tid % kResHalf; l < l1; l += kResHalf) {
                         const int item = B.list[l], e = item >> 5, j = item & 31, cell = B.cell[e];
                         if (walls && a.wall[cell]) continue;  // wall nodes hold f = 0 (fluids.jl:154)
-                        const int ci[3] = {s_lat[0][j], s_lat[1][j], s_lat[2][j]};
+                        const int ci[2] = {s_lat[0][j], s_lat[1][j]};
                         const double rhoL = B.rho[e], gi = (double)B.gi[l];
                         double v = gi;  // halfway bounce-back: f_j(x) = f*_i(x)
                         if (a.uw) {     // moving walls (fluids.jl:168-174)
                             const int q = source(item);
-                            const double dot = -(ci[0] * a.uw[q] + ci[1] * a.uw[a.g.N + q] +
-                                                 (D == 3 ? ci[2] * a.uw[2 * a.g.N + q] : 0.0));
-                            v += 6.0 * rhoL * dot;
+                            v += 6.0 * rhoL * -(ci[0] * a.uw[q] + ci[1] * a.uw[a.g.N + q]);
                         }
                         if (sP.dirlinks >> j & 1u) {
                             v += 6.0 * rhoL * -B.cu[l];
                             if (sP.coupleF || sP.coupleT || sP.recordF) {
-                                const double Xc[3] = {coord(e, 0, 0), coord(e, 1, 0), D == 3 ? coord(e, 2, 0) : 0.0};
-                                resident_exchange<D>(a, sP, ci, Xc, gi, s_w[j], v, acc);
+                                const double Xc[2] = {coord(e, 0, 0), coord(e, 1, 0)};
+                                resident_exchange(a, sP, ci, Xc, gi, s_w[j], v, acc);
                             }
                         }
                         dst[j * a.g.N + cell] = SS::enc((R)v, R(a.scale));
                     }
                     // as fixup_body: butterfly inside warps, then the warps in order
 #pragma unroll
-                    for (int k = 0; k < (D == 2 ? 4 : 6); ++k) {
-                        if (D == 2 && k == 2) continue;  // (2D: two force components and one torque)
+                    for (int k = 0; k < 4; ++k) {
+                        if (k == 2) continue;
                         for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
                         if (lane == 0) s_red[warp][k] = acc[k];
                     }
@@ -858,7 +813,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                 if (tid < 6 * kHalves && c0 + tid / 6 < nch) {
                     const int h = tid / 6, k = tid % 6;
                     double sum = 0.0;
-                    if (D == 3 || (k < 4 && k != 2))
+                    if (k < 4 && k != 2)
                         for (int w = 0; w < kResHalf / 32; ++w) sum += s_red[h * (kResHalf / 32) + w][k];
                     s_part[c0 + h][k] = sum;
                 }
