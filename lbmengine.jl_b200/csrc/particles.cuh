@@ -51,8 +51,9 @@ struct ParticleArgs {
 };
 
 // the updated record P (in shared memory) back to global memory, and into the
-// history lbm_adjoint keeps; every thread of the CTA, after a barrier
-__device__ __forceinline__ void store_record(const ParticleArgs& a, int p, const ParticleDev& P) {
+// history lbm_adjoint keeps; every thread of the CTA, after a barrier.  err: the
+// error word as thread 0 found it
+__device__ __forceinline__ void store_record(const ParticleArgs& a, int p, const ParticleDev& P, int err = 0) {
     const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&P);
     unsigned long long* dst = reinterpret_cast<unsigned long long*>(a.parts + p);
     unsigned long long* rec =
@@ -61,7 +62,7 @@ __device__ __forceinline__ void store_record(const ParticleArgs& a, int p, const
         dst[k] = src[k];
         if (rec) rec[k] = src[k];
     }
-    if (rec && threadIdx.x == 0 && *(volatile const int*)a.err) atomicCAS(a.first_err, INT_MAX, P.rec_tick);
+    if (rec && threadIdx.x == 0 && err) atomicCAS(a.first_err, INT_MAX, P.rec_tick);
 }
 
 // publish particle p's solid box for the far/near split of the bulk pass
@@ -655,10 +656,11 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
     static_assert(sizeof(ParticleDev) % 8 == 0, "ParticleDev is copied in 8-byte words");
     const unsigned long long* gsrc = reinterpret_cast<const unsigned long long*>(a.parts + p);
     unsigned long long* sdst = reinterpret_cast<unsigned long long*>(&sP);
+    const int err = a.rec && threadIdx.x == 0 ? *(volatile const int*)a.err : 0;  // in flight with the record
     for (int k = threadIdx.x; k < (int)(sizeof(ParticleDev) / 8); k += blockDim.x) sdst[k] = gsrc[k];
     __syncthreads();
     particles_core<L, LK>(a, p, sP);
-    store_record(a, p, sP);
+    store_record(a, p, sP, err);
     if (threadIdx.x == 0) publish_box(a, p, sP);
 }
 
