@@ -132,10 +132,12 @@ typedef struct lbm_config {
 #define LBM_RULES_GPU_MODULE 0
 #define LBM_RULES_CPU_MODULE 1
 
-/* Kernel schedule of a tick.  Results do not depend on it (the per-node
- * arithmetic is the same).
- *   AUTO        (default) small 2D models with FP32 or FP64 storage: many
- *               ticks in one launch; every other model: STREAM
+/* Kernel schedule of a tick.  The arithmetic of a node and of a link is the
+ * same in all of them; the FP64 rounding of the particles' sums and updates may
+ * differ (their state by 1e-12 of itself, and where that changes how a stored
+ * population rounds, the population by a unit in the last place).
+ *   AUTO        (default) small 2D models with FP32 or FP64 storage, in calls of
+ *               more than a few ticks: many ticks in one launch; else STREAM
  *   STREAM      bulk -> fix-up in stream order, particle update on a side
  *               stream overlapping the next bulk pass; with many particles
  *               the fix-up too, except for its stores
@@ -519,7 +521,8 @@ int lbm_adjoint(lbm_handle* h, const lbm_adjoint_spec* spec, lbm_adjoint_result*
 
 /* Allocation-free stepping.  No counterpart in the reference.
  *
- * Same ticks and results as lbm_step, for callers that must not allocate
+ * Same ticks as lbm_step, with the same bits as in stream order
+ * (LBM_SCHEDULE_STREAM), for callers that must not allocate
  * device memory once their run has started: codes that reserve all device
  * memory up front (another library's memory pool, a fixed per-process budget)
  * and real-time or embedded hosts whose policy forbids allocation after
@@ -548,9 +551,9 @@ int lbm_step_noalloc(lbm_handle* h, int64_t nsteps);
 
 /* lbm_destroy waits for the handle's queued work and gives its device
  * buffers back.  The library keeps freed device blocks (up to 4 GiB in the
- * process, the ones freed longest ago giving way) for later allocations of the same size, so a model built after
- * another does not pay cudaMalloc again; the kept blocks go back to the
- * driver when a cudaMalloc fails. */
+ * process, the ones freed longest ago giving way) for later allocations of the
+ * same size, so a model built after another does not pay cudaMalloc again; the
+ * kept blocks go back to the driver when a cudaMalloc fails. */
 const char* lbm_last_error(lbm_handle* h);
 const char* lbm_last_global_error(void);
 void lbm_destroy(lbm_handle* h);

@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(LIST ? kListThreads : kFixThreads, 512 / (LIST
 // follow the bulk pass is the store of the listed values, a few microseconds
 // (k_fixup_store).  Only the chain store -> next bulk pass stays on the main
 // stream.  64 particles of r = 6 in 192^3 (BF16):
-// 132 -> 107-112 us per tick; 128 D2Q9 replicas of 64^2 to 256^2 62 -> 47.6.
+// 132 -> 112 us per tick; 128 D2Q9 replicas of 64^2 to 256^2 62 -> 47.6.
 // ---------------------------------------------------------------------------
 constexpr int kStoreThreads = 256;
 

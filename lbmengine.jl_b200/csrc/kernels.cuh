@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(B, bulk_threads_per_sm<L, ST, SR, X2>() / B) k
     // FP32: the last three fifths of the pass store with the default policy,
     // so that L2 keeps those lines for the next pass (128^3 tick: 51.3 us with
     // none, 50.5 with two fifths, 49.4 with three, 50.2 with four, 51.6 with
-    // all); the issue-bound 2-byte passes measured slower with it
+    // all); the 2-byte passes measured slower with it
     const bool keep = Store<ST>::bytes == 4 && (long long)blockIdx.x * 5 >= tiles * 2;
     bulk_v4_tile<L, ST, TRT, B, SR, X2>(a, a.reverse ? tiles - 1 - (long long)blockIdx.x : (long long)blockIdx.x, s_ex,
                                         keep);

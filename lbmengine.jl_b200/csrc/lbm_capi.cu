@@ -570,8 +570,9 @@ double bulk_us(const lbm_handle* h) { return 2.0 * h->q * storage_bytes(h->stora
 // CTAs per particle of the fix-up beside the bulk pass.  A CTA takes up to
 // 20 us per chunk and the particle update behind it about 30: up to four
 // chunks in turn where the bulk pass hides both, because more CTAs at once
-// only take registers from it (64 particles of r = 6 in 192^3 BF16:
-// 3 / 4 / 6 / 18 CTAs per particle 107.1 / 106.5 / 107.4 / 110.8 us per tick; 32 of r = 8 in 128^3 FP32: 6 / 19 CTAs 92.8 / 59.7 us).
+// only take registers from it (64 slow particles of r = 6 in 192^3 BF16:
+// 3 / 4 / 6 / 18 CTAs per particle 107.1 / 106.5 / 107.4 / 110.8 us per tick; 32 of
+// r = 8 in 128^3 FP32: 6 / 19 CTAs 92.8 / 59.7 us).
 int list_ctas(const lbm_handle* h) {
     const int turns = (int)std::min(4.0, std::max(1.0, std::floor((bulk_us(h) - 30.0) / 20.0)));
     return (list_chunks(h) + turns - 1) / turns;
@@ -870,7 +871,8 @@ int slot_list(lbm_handle* h) {
 // fix-up -> particle update has to fit into the bulk pass, and a launch is
 // added.  So: more chunks than one wave, and a bulk pass (its bytes at 6.5 TB/s)
 // no shorter than the particle update (18 us + 0.095 us r^2 in 3D, 10 us in
-// 2D), or many waves of small particles.  Ticks in us, behind / beside:
+// 2D), or many waves of small particles.  Ticks in us, behind / beside (slow
+// particles, whose links are seldom rebuilt):
 //   D3Q19  192^3 BF16, 64 of r = 6 125 / 107;  27 of r = 6 111 / 100
 //          128^3 FP32, 8 of r = 8 (152 chunks) 57.1 / 57.8;  16 66.6 / 64.4;  32 76.7 / 60.0;
 //                      8 of r = 16 77.7 / 69.4;  1 of r = 20 (122 chunks) 61.8 / 66.5;  1 of r = 32 101 / 103

@@ -18,13 +18,17 @@
 //                 next tick run behind the barrier.
 // Where the geometry changes (one tick in tens), the CTA rebuilds it, the slot
 // list and pmask before it arrives, and the others wait.
-// The arithmetic of a node, a link slot and a particle, and the order of the
-// FP64 sums, are those of k_bulk, k_fixup and k_particles: the populations are
-// equal bit for bit.
+// The operations of a node, a link slot and a particle, and the order of the
+// FP64 sums, are those of k_bulk, k_fixup and k_particles.  The compiler may
+// contract the particle's here otherwise than there: its state agrees with the
+// stream schedule's to 1e-12 of itself while the stored populations round
+// alike, and these to a unit in the last place (1e-7 FP32, 1e-13 FP64; tested).
 //
-// Measured with a squirmer, per tick, against the stream schedule: 64^2 FP32
-// 3.4 us (9.2), 256 x 128 FP64 4.2 (9.9), 201 x 65 FP64 with walls 4.2 (11.1),
-// 512 x 256 FP32 4.4 (9.7), 724^2 FP32 8.9 (11.2).  The chain that bounds it: barrier and fence 1.0,
+// Measured in calls of 2,000 ticks, us per tick, against the stream schedule:
+// with a squirmer 64^2 FP32 3.4 (9.0), 256 x 128 FP64 4.0 (9.5), 201 x 65 FP64 with
+// walls 4.2 (9.6), 512 x 256 FP32 4.0 (9.4), 724^2 FP32 8.9 (10.2); with a bead
+// 201 x 65 FP64 with walls 3.8 (9.4), with a moving lid 5.0 (9.6); faster swimmers, whose
+// geometry changes more often, 0.2-0.6 more.  The chain that bounds it: barrier and fence 1.0,
 // link nodes 0.8, slots and their sums 0.7, the verdict on the geometry 0.4 us.
 // (Two barriers per tick, with the slots stored between them over the pushes,
 // took 3.4 to 5.6 us for the same grids.)
