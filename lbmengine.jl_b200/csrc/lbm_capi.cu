@@ -129,7 +129,8 @@ struct lbm_handle {
     int res_ctas = -1;                  // CTAs of the launch; 0: does not apply, -1: not looked up yet
     int res_cluster = 0;                // CTAs per cluster; 0: one cooperative grid
     bool res_ready = false;             // the jobs below are current
-    int64_t res_hold = 0, res_wait = 0; // ticks left in stream order after a launch that ended early, and of the last such wait
+    int64_t res_hold = 0;               // ticks left in stream order after a launch that ended early
+    int64_t res_wait = 0;               // and how many there were
     ResidentJob* d_rjobs = nullptr;     // [2]: by the buffer the first tick reads
     unsigned *d_pmask = nullptr, *d_wmask = nullptr;
     int* d_rsync = nullptr;             // barrier counter and last phase, then the particles' boxes
@@ -882,9 +883,11 @@ int slot_list(lbm_handle* h) {
 //   D2Q9   2048^2 FP32, 250 of r = 20 103 / 66;  1024^2 FP32, 250 of r = 8 28.5 / 23.5
 // D3Q27's list CTAs hold more registers and memory, and hold the bulk pass up
 // where there are few of them beside a long pass, with FP64 storage always:
-//   D3Q27  FP32  27 of r = 6 (297 chunks) 96^3 53.5 / 61.2, 128^3 98.9 / 96.4, 160^3 168 / 193;  160^3, 2 of r = 25 (380) 171 / 189
-//                64 of r = 5 (512) 96^3 65.0 / 61.6;  128^3, 8 of r = 16 115 / 94;  160^3, 64 of r = 8 210 / 203
-//          FP16  27 of r = 6 128^3 61.5 / 63.9, 160^3 105 / 93.6;  160^3, 2 of r = 25 109 / 98;  128^3, 64 of r = 6 77.4 / 63.1
+//   D3Q27  FP32  27 of r = 6 (297 chunks) 96^3 53.5 / 61.2, 128^3 98.9 / 96.4, 160^3 168 / 193;
+//                160^3, 2 of r = 25 (380) 171 / 189;  96^3, 64 of r = 5 (512) 65.0 / 61.6;
+//                128^3, 8 of r = 16 115 / 94;  160^3, 64 of r = 8 210 / 203
+//          FP16  27 of r = 6 128^3 61.5 / 63.9, 160^3 105 / 93.6;  160^3, 2 of r = 25 109 / 98;
+//                128^3, 64 of r = 6 77.4 / 63.1
 //          FP64  128^3, 27 of r = 6 172 / 287;  96^3, 64 of r = 5 107 / 114;  160^3, 64 of r = 8 359 / 418
 // There: none with FP64, else one and a half waves, or with 2-byte storage a
 // bulk pass of two particle updates.
@@ -996,8 +999,10 @@ long long resident_nodes(const lbm_handle* h, int64_t nsteps) {
 // blocking read) and gains some microseconds per tick.  us per call, resident /
 // stream (FP32; FP64 alike):
 //   fluid 64^2                    2 ticks 26 / 19, 4 26 / 25, 8 38.6 / 38.6, 10 39 / 42
-//   walls, 11,000 nodes           1 28 / 17, 2 29 / 27, 3 29 / 28, 5 33 / 39; 99,000 nodes 4 41 / 37, 8 53 / 51, 10 57 / 68
-//   one particle, r = 3           1 29 / 25, 2 33 / 39; r = 14 2 41 / 39, 3 41 / 52; r = 28 3 53 / 52, 4 54 / 50, 5 65 / 65, 6 67 / 77
+//   walls, 11,000 nodes           1 28 / 17, 2 29 / 27, 3 29 / 28, 5 33 / 39;
+//          99,000 nodes           4 41 / 37, 8 53 / 51, 10 57 / 68
+//   one particle, r = 3           1 29 / 25, 2 33 / 39; r = 14 2 41 / 39, 3 41 / 52;
+//                 r = 28          3 53 / 52, 4 54 / 50, 5 65 / 65, 6 67 / 77
 //   eight particles, 11,520 nodes 1 42 / 25, 3 52 / 52, 5 62 / 66; 490,000 nodes 5 87 / 75, 10 131 / 139
 int64_t resident_min_ticks(const lbm_handle* h) {
     const size_t np = h->hparts.size();
