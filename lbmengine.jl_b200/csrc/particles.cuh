@@ -52,7 +52,7 @@ struct ParticleArgs {
 
 // the updated record P (in shared memory) back to global memory, and into the
 // history lbm_adjoint keeps; every thread of the CTA, after a barrier.  err: the
-// error word as thread 0 found it
+// error word, with a history
 __device__ __forceinline__ void store_record(const ParticleArgs& a, int p, const ParticleDev& P, int err = 0) {
     const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&P);
     unsigned long long* dst = reinterpret_cast<unsigned long long*>(a.parts + p);
@@ -62,7 +62,7 @@ __device__ __forceinline__ void store_record(const ParticleArgs& a, int p, const
         dst[k] = src[k];
         if (rec) rec[k] = src[k];
     }
-    if (rec && threadIdx.x == 0 && err) atomicCAS(a.first_err, INT_MAX, P.rec_tick);
+    if (err && a.mode == 0 && threadIdx.x == 0) atomicCAS(a.first_err, INT_MAX, P.rec_tick);
 }
 
 // publish particle p's solid box for the far/near split of the bulk pass
@@ -656,7 +656,8 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a, const int 
     static_assert(sizeof(ParticleDev) % 8 == 0, "ParticleDev is copied in 8-byte words");
     const unsigned long long* gsrc = reinterpret_cast<const unsigned long long*>(a.parts + p);
     unsigned long long* sdst = reinterpret_cast<unsigned long long*>(&sP);
-    const int err = a.rec && threadIdx.x == 0 ? *(volatile const int*)a.err : 0;  // in flight with the record
+    int err = 0;
+    if (a.rec) err = *(volatile const int*)a.err;  // in flight with the record
     for (int k = threadIdx.x; k < (int)(sizeof(ParticleDev) / 8); k += blockDim.x) sdst[k] = gsrc[k];
     __syncthreads();
     particles_core<L, LK>(a, p, sP);
